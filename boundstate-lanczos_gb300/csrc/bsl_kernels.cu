@@ -173,34 +173,114 @@ __global__ void k_potential_coulomb(const double* xg, const double* yg, const do
   v2[t] = v;
 }
 
-// one thread per (point, theta_a, phi_b): both phi halves
-__global__ void k_potential_alavi(AtomSet atoms, const double* xg, const double* yg, const double* zg, int nx, int ny,
-                                  long long npts, int nab, const double* hdir, const double* cm, double ceiling,
-                                  double* v1, double* v2) {
-  __shared__ double sxyz[3 * kMaxAtoms], sq[kMaxAtoms];
+// RN(k / RN(sqrt(r2))), the two correctly rounded FP64 operations, in 6 FP64
+// instructions.  The FP64 pipe executes 2 lanes a clock and SM, the FP32 and
+// integer pipes 128, so the reciprocal root y is refined to ~2^-45 in FP32 (the
+// residual 1 - r2 y0^2 of the hardware's estimate with the error of every
+// product) and put together with integer operations; one FP64 residual each
+// then gives the root and the quotient to ~2^-89 before their final rounding
+// (Markstein, IBM J. Res. Dev. 34, 1990).  Sets bad for r2 outside [2^-60, 2^62).
+__device__ __forceinline__ double quotient_root(double k, double r2, bool& bad) {
+  const unsigned int hi = (unsigned int)__double2hiint(r2), lo = (unsigned int)__double2loint(r2);
+  bad = bad || (hi - 0x3C300000u) >= 0x07A00000u;
+  // r2 = a + b: the leading 24 bits and the other 29, rounded
+  const float a = __uint_as_float(__funnelshift_l(lo, hi, 3) - 0xC0000000u);
+  const float b = __fmul_rn((float)(lo & 0x1FFFFFFFu), __uint_as_float(((hi >> 20) - 948u) << 23));
+  const float y0 = rsqrtf(a);
+  const float p = __fmul_rn(y0, y0), pe = __fmaf_rn(y0, y0, -p);
+  const float t = __fmaf_rn(-b, p, __fmaf_rn(-a, pe, __fmaf_rn(-a, p, 1.f)));
+  const float c = __fmul_rn(__fmul_rn(y0, t), __fmaf_rn(0.375f, t, 0.5f));
+  // y = y0 + c, c as a fixed-point number of units 2^-50 of y0's binade
+  const unsigned int yb = __float_as_uint(y0);
+  const int n = __float2int_rn(__fmul_rn(c, __uint_as_float((304u - (yb >> 23)) << 23)));
+  long long m = ((long long)(yb & 0x7FFFFFu) << 29) + ((long long)n << 2);
+  // y in the binade below or above y0's: its mantissa in that binade's units
+  if ((unsigned int)(m >> 32) > 0xFFFFFu) m = m < 0 ? 2 * m : (m + (1ll << 52)) >> 1;
+  const long long ybits = ((long long)((yb >> 23) + 896u) << 52) + m;
+  const double y = __longlong_as_double(ybits), half_y = __longlong_as_double(ybits - (1ll << 52));
+  const double s0 = __dmul_rn(r2, y);
+  const double s = fma(fma(-s0, s0, r2), half_y, s0);
+  const double q0 = __dmul_rn(k, y);
+  return fma(fma(-q0, s, k), y, q0);
+}
+
+// One thread per point, theta_a and kPhis values of phi_b, both phi halves.
+// Bound by the FP64 pipe: the two H positions of a node and of its mirror image
+// under phi -> 2 pi - phi share their coordinates, and all of a theta their z,
+// which leaves 4.3 operations for a squared distance, 6 for the term and 1 to
+// add it, against 29 with one thread per node and the compiler's square root
+// and division: 303 instead of 698 ms at 41^3, 30 x 60 nodes, 60 sites (267 ms
+// at the pipe's rate).  The results are the same bits.
+constexpr int kPhis = 3;
+__global__ void __launch_bounds__(kThreads) k_potential_alavi(AtomSet atoms, const double* xg, const double* yg,
+                                                              const double* zg, int nx, int ny, long long npts,
+                                                              int na, int nb, const double* hdir, const double* cm,
+                                                              double ceiling, double* v1, double* v2) {
+  __shared__ double sxyz[3 * kMaxAtoms], sq[kMaxAtoms], skq[kMaxAtoms];
   for (int i = threadIdx.x; i < atoms.n; i += blockDim.x) {
     sxyz[3 * i] = atoms.xyz[3 * i];
     sxyz[3 * i + 1] = atoms.xyz[3 * i + 1];
     sxyz[3 * i + 2] = atoms.xyz[3 * i + 2];
     sq[i] = atoms.q[i];
+    skq[i] = __dmul_rn(__dmul_rn(kCoulombK, atoms.q_h), atoms.q[i]);
   }
   __syncthreads();
+  const int nbg = (nb + kPhis - 1) / kPhis, nab = na * nb;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npts * nab) return;
-  const long long p = t / nab;
-  const int ab = (int)(t % nab);
+  if (t >= npts * na * nbg) return;
+  const long long p = t / (na * nbg);
+  const int ag = (int)(t - p * (na * nbg)), a = ag / nbg, b0 = (ag - a * nbg) * kPhis;
   const int i = (int)(p % nx), j = (int)((p / nx) % ny), k = (int)(p / ((long long)nx * ny));
-  const double x = xg[i], y = yg[j], z = zg[k];
-  const double hx = hdir[3 * ab], hy = hdir[3 * ab + 1], hz = hdir[3 * ab + 2];
-  const double c = cm[p];
+  const double x = xg[i], y = yg[j], z = zg[k], c = cm[p];
+  const double hz = hdir[3 * (a * nb) + 2];  // the same for every phi
+  const double zp = __dadd_rn(z, hz), zm = __dsub_rn(z, hz);
+  double xp[kPhis], xm[kPhis], yp[kPhis], ym[kPhis];
+  double e[kPhis][2][2];  // [phi][half][H at +h, at -h]
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const double hyh = half ? -1.0 * hy : hy;
-    double v = coulomb(sxyz, sq, atoms.n, atoms.q_h, __dadd_rn(x, hx), __dadd_rn(y, hyh), __dadd_rn(z, hz));
-    v = __dadd_rn(v, coulomb(sxyz, sq, atoms.n, atoms.q_h, __dsub_rn(x, hx), __dsub_rn(y, hyh), __dsub_rn(z, hz)));
-    v = __dadd_rn(v, c);
-    if (v >= ceiling) v = ceiling;
-    (half ? v2 : v1)[t] = v;
+  for (int u = 0; u < kPhis; ++u) {
+    const double* h = hdir + 3 * (a * nb + min(b0 + u, nb - 1));
+    xp[u] = __dadd_rn(x, h[0]);
+    xm[u] = __dsub_rn(x, h[0]);
+    yp[u] = __dadd_rn(y, h[1]);
+    ym[u] = __dsub_rn(y, h[1]);
+    e[u][0][0] = e[u][0][1] = e[u][1][0] = e[u][1][1] = 0.0;
+  }
+  bool bad = false;
+  for (int w = 0; w < atoms.n; ++w) {
+    const double sx = sxyz[3 * w], sy = sxyz[3 * w + 1], sz = sxyz[3 * w + 2], kq = skq[w];
+    auto square = [](double s, double q) {
+      const double d = __dsub_rn(s, q);
+      return __dmul_rn(d, d);
+    };
+    const double zp2 = square(sz, zp), zm2 = square(sz, zm);
+#pragma unroll
+    for (int u = 0; u < kPhis; ++u) {
+      const double xp2 = square(sx, xp[u]), xm2 = square(sx, xm[u]);
+      const double yp2 = square(sy, yp[u]), ym2 = square(sy, ym[u]);
+      // half 0: H at (x + hx, y + hy, z + hz) and (x - hx, y - hy, z - hz); half 1: hy changes sign
+      auto add = [&](double& sum, double dx2, double dy2, double dz2) {
+        sum = __dadd_rn(sum, quotient_root(kq, __dadd_rn(__dadd_rn(dx2, dy2), dz2), bad));
+      };
+      add(e[u][0][0], xp2, yp2, zp2);
+      add(e[u][0][1], xm2, ym2, zm2);
+      add(e[u][1][0], xp2, ym2, zp2);
+      add(e[u][1][1], xm2, yp2, zm2);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kPhis; ++u) {
+    if (b0 + u >= nb) break;
+    const int ab = a * nb + b0 + u;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (bad) {  // a site at or absurdly near or far from an H atom: the plain operations
+        e[u][half][0] = coulomb(sxyz, sq, atoms.n, atoms.q_h, xp[u], half ? ym[u] : yp[u], zp);
+        e[u][half][1] = coulomb(sxyz, sq, atoms.n, atoms.q_h, xm[u], half ? yp[u] : ym[u], zm);
+      }
+      double v = __dadd_rn(__dadd_rn(e[u][half][0], e[u][half][1]), c);
+      if (v >= ceiling) v = ceiling;
+      (half ? v2 : v1)[p * nab + ab] = v;
+    }
   }
 }
 
@@ -726,11 +806,10 @@ int dev_potential_alavi(bsl_handle* h) {
   }
   AtomSet atoms{dxyz, dq, dis_o, natoms, h->cage.q_h2_h, h->cage.q_h2_cm, h->cage.lj_a, h->cage.lj_b};
   const long long N = t.npts;
-  const int nab = t.na * t.nb;
   double* cm = d.ukin;  // scratch of >= N doubles
   k_site_energy<<<grid_for(N), kThreads, 0, d.stream>>>(atoms, dx, dy, dz, t.nx, t.ny, N, atoms.q_cm, 1, cm);
-  k_potential_alavi<<<grid_for(N * nab), kThreads, 0, d.stream>>>(atoms, dx, dy, dz, t.nx, t.ny, N, nab, dh, cm,
-                                                                  h->p.ceiling_potential, d.v1, d.v2);
+  k_potential_alavi<<<grid_for(N * t.na * ((t.nb + kPhis - 1) / kPhis)), kThreads, 0, d.stream>>>(
+      atoms, dx, dy, dz, t.nx, t.ny, N, t.na, t.nb, dh, cm, h->p.ceiling_potential, d.v1, d.v2);
   e = cudaGetLastError();
   cudaError_t e2 = cudaStreamSynchronize(d.stream);
   cleanup();
