@@ -330,6 +330,8 @@ void free_device(DeviceState& d) {
   if (d.vpair) cudaFree(d.vpair);
   if (d.kxy_slices) cudaFree(d.kxy_slices);
   if (d.kz_slices) cudaFree(d.kz_slices);
+  if (d.tx_slices32) cudaFree(d.tx_slices32);
+  if (d.tz_slices32) cudaFree(d.tz_slices32);
   if (d.jdev) cudaFree(d.jdev);
   if (d.vb16) cudaFree(d.vb16);
   if (d.vscale) cudaFree(d.vscale);
@@ -434,6 +436,11 @@ int hv_prep(const bsl_hv_params* params, const Cage* cage, bsl_handle** out) {
     if ((rc = upload(&d.kxy_slices, sl, "Tx"))) return bail(rc);
     kinetic_smem_image(t.tz, t.nz, false, &sl, &d.e_tz);
     if ((rc = upload(&d.kz_slices, sl, "Tz"))) return bail(rc);
+    std::vector<float> sf;
+    kinetic_slices_f32(t.tx, t.nx, &sf);
+    if ((rc = upload(&d.tx_slices32, sf, "Tx"))) return bail(rc);
+    kinetic_slices_f32(t.tz, t.nz, &sf);
+    if ((rc = upload(&d.tz_slices32, sf, "Tz"))) return bail(rc);
     h->kinetic_engine = BSL_KIN_TENSOR;
   }
   if ((rc = upload(&d.rot, t.rot, "rotor"))) return bail(rc);

@@ -99,6 +99,7 @@ struct DeviceState {
   // exponents, for the tensor-core kinetic
   uint16_t *kxy_slices = nullptr, *kz_slices = nullptr;
   int e_txy = 0, e_tz = 0;
+  float *tx_slices32 = nullptr, *tz_slices32 = nullptr;  // the slices as FP32 integers (bsl_small.cu)
   int kin_grid_xy = 0, kin_grid_z = 0;  // persistent grid sizes
   double* rot = nullptr;  // [nn]
   // potential grid V(p, a, b) for phi_b and 2pi - phi_b, p in vector order
@@ -225,6 +226,11 @@ int launch_kin_z_mixed(bsl_handle* h, const float* v, cudaStream_t s);
 void kinetic_smem_image(const std::vector<double>& T, int n, bool with_zero_tiles, std::vector<uint16_t>* image,
                         int* e_t);
 bool kinetic_tc_supported(const Tables& t);
+void kinetic_slices_f32(const std::vector<double>& T, int n, std::vector<float>* out);
+// small grids: the three contractions in one launch (bsl_small.cu); fin_count:
+// block totals of a deferred beta to finish
+bool kin_small_supported(const bsl_handle* h);
+int launch_kin_small(bsl_handle* h, const float2* v, int fin_count, cudaStream_t s);
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 int launch_kin_z_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 // grouped tensor-core kinetic over several problems: per-problem argument

@@ -704,9 +704,12 @@ int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, 
 // mixed-precision kinetic stages by the selected engine: the tensor-core engine
 // reads v as double-float pairs, the CUDA-core engine its FP32 copy
 int launch_kin_xy(bsl_handle* h, const float2* vpair, cudaStream_t s) {
+  if (h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h))  // all three contractions
+    return launch_kin_small(h, vpair, h->defer_reductions ? deferred_beta_count(h) : 0, s);
   return h->kinetic_engine == BSL_KIN_TENSOR ? launch_kin_xy_tc(h, vpair, s) : launch_kin_xy_mixed(h, h->d.v32, s);
 }
 int launch_kin_z(bsl_handle* h, const float2* vpair, cudaStream_t s) {
+  if (h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)) return BSL_OK;
   return h->kinetic_engine == BSL_KIN_TENSOR ? launch_kin_z_tc(h, vpair, s) : launch_kin_z_mixed(h, h->d.v32, s);
 }
 
@@ -1169,8 +1172,10 @@ const char* dev_stage_name(bsl_handle* h, int i) {
   const bool mixed = h->precision == BSL_PREC_MIXED;
   static const char* n64[4] = {"k_kin_xy_f64", "k_kin_z_f64", "k_vapply<NN,double>", "k_update_fold"};
   static const char* nmx[4] = {"k_kin_xy_split", "k_kin_z_split", "k_vstream<NN>", "k_update_pair"};
+  static const char* nts[2] = {"k_kin_small", "(in k_kin_small)"};
   static const char* ntc[4] = {"k_kin_xy_tc", "k_kin_z_tc", "k_vstream<NN>", "k_update_stream"};
   if (!mixed) return n64[i];
+  if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)) return nts[i];
   if (fused_iterations(h) && i >= 2)
     return i == 2 ? "k_vapply_light<NN>" : h->vformat == BSL_VFMT_GAUNT ? "k_vstream<NN,coefficients,update>"
                                                                         : "k_vstream<NN,fp32,update>";

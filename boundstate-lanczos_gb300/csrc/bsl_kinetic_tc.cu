@@ -51,13 +51,12 @@
 
 #include "bsl_device.cuh"
 #include "bsl_internal.h"
+#include "bsl_slices.cuh"
 #include "bsl_tc.cuh"
 
 namespace bsl {
 namespace {
 
-constexpr int kVS = 4;                        // slices of v
-constexpr int kTS = 4;                        // slices of T
 constexpr uint32_t kTile = 64 * 128;          // 8 KiB: 64 rows x 64 FP16, one 128-byte swizzled row each
 constexpr uint32_t kPlaneSlices = kVS * kTile;  // the v slices of one plane, contiguous
 constexpr uint32_t kStage = 2 * kPlaneSlices;   // v slices of a plane pair: [plane][slice] tiles
@@ -103,36 +102,9 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// exponent e with max|x| 2^-e in [0.5, 1]; 0 for an all-zero plane
-__device__ __forceinline__ int plane_exponent(float maxabs) {
-  if (!(maxabs > 0.f)) return 0;
-  return max(-100, ilogbf(maxabs) + 1);
-}
-
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((min(max(e, -126), 127) + 127) << 23); }
-
-// Four 9-bit slices of a double-float value already scaled to |y| < 256 (hi and
-// lo multiplied by the same power of two): y = a1 + 2^-9 a2 + 2^-18 a3 +
-// 2^-27 a4 + O(2^-28), each a an integer in [-256, 256].  Every step is exact
-// except the last rounding.
-__device__ __forceinline__ void slice4(float yh, float yl, float (&a)[kVS]) {
-  a[0] = rintf(yh);
-  float r = __fmul_rn(__fadd_rn(__fsub_rn(yh, a[0]), yl), 512.f);
-  a[1] = rintf(r);
-  r = __fmul_rn(__fsub_rn(r, a[1]), 512.f);
-  a[2] = rintf(r);
-  r = __fmul_rn(__fsub_rn(r, a[2]), 512.f);
-  a[3] = rintf(r);
-}
-
-// the four class accumulators of 8 consecutive columns combined into
-// double-float pairs and multiplied by `scale` (a power of two).  The classes
-// are exact integers below 2^24: the head is c0 + 2^-9 c1 with its rounding
-// error, the tail collects that error and the two smaller classes (its own
-// rounding is ~2^-33 of the head); the pair is left unnormalised (|lo| may
-// slightly exceed half an ulp of hi), which the double-float additions accept.
-// With fewer than four slices the classes at and above `nslices` were never
-// written and are taken as zero.
+// the four class accumulators of 8 consecutive columns as double-float pairs
+// times `scale` (combine_classes).  With fewer than four slices the classes at
+// and above `nslices` were never written and are taken as zero.
 __device__ __forceinline__ void load_pairs8(uint32_t taddr, float scale, int nslices, float2 (&out)[8]) {
   float c0[8], c1[8], c2[8], c3[8];
   tc::tmem_ld8_nowait(taddr, c0);
@@ -149,12 +121,7 @@ __device__ __forceinline__ void load_pairs8(uint32_t taddr, float scale, int nsl
     }
   }
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    float h, e;
-    two_sum(c0[u], __fmul_rn(c1[u], 0x1p-9f), h, e);
-    const float l = __fmaf_rn(c3[u], 0x1p-27f, __fmaf_rn(c2[u], 0x1p-18f, e));
-    out[u] = make_float2(__fmul_rn(h, scale), __fmul_rn(l, scale));
-  }
+  for (int u = 0; u < 8; ++u) out[u] = combine_classes(c0[u], c1[u], c2[u], c3[u], scale);
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -551,6 +518,23 @@ void kinetic_smem_image(const std::vector<double>& T, int n, bool with_zero_tile
         r = (r - b) * 512.0;
       }
     }
+}
+
+// The same slices as FP32 integers, [slice][i][q], for the small-grid kernel.
+void kinetic_slices_f32(const std::vector<double>& T, int n, std::vector<float>* out) {
+  double m = 0.0;
+  for (double x : T) m = std::max(m, std::fabs(x));
+  int e = 0;
+  if (m > 0.0) std::frexp(m, &e);
+  out->assign((size_t)kTS * n * n, 0.f);
+  for (int i = 0; i < n * n; ++i) {
+    double r = std::ldexp(T[i], 8 - e);
+    for (int l = 0; l < kTS; ++l) {
+      const double b = std::nearbyint(r);
+      (*out)[(size_t)l * n * n + i] = (float)b;
+      r = (r - b) * 512.0;
+    }
+  }
 }
 
 bool kinetic_tc_supported(const Tables& t) { return t.nx <= 64 && t.ny <= 64 && t.nz <= 64 && t.tx == t.ty; }

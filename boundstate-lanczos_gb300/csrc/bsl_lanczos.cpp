@@ -829,7 +829,11 @@ int bsl_stage_times(bsl_handle* h, int iters, double* ms, const char** names) {
   return check_status(h);
 }
 
-int bsl_launches_per_iteration(const bsl_handle* h) { return h ? 4 : -1; }
+int bsl_launches_per_iteration(const bsl_handle* h) {
+  if (!h) return -1;
+  const bool one = h->precision == BSL_PREC_MIXED && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h);
+  return one ? 3 : 4;  // kinetic in one launch or two
+}
 
 int bsl_debug_inject_timeout(bsl_handle* h, int kernel_mask) {
   if (!h) return fail(BSL_ERR_STATE, "null handle");
