@@ -307,7 +307,7 @@ int launch_light_group(const void* d_args, const int4* d_work, int nctas, cudaSt
 int launch_vstream_group(const void* d_args, const int4* d_work, int nctas, cudaStream_t s);
 // the potential stream's arguments for one problem (mode 2, j from the device counter)
 StreamArgs vstream_args(bsl_handle* h, const double* v, double* out);
-int launch_vapply_f64(const double* vb, dim3 g, cudaStream_t s, int nn, const double* v, const double* uk,
+int launch_vapply_f64(const double* vb, cudaStream_t s, int nn, const double* v, const double* uk,
                       const double* rot, double* out, long long N, int mode, double* partials, unsigned int* counter,
                       double* scalars, double* hist, int j, long long dpk);
 

@@ -369,47 +369,35 @@ __global__ void k_vblocks(BlockTables bt, const double* v1, const double* v2, lo
 // ---------------------------------------------------------------------------
 // kinetic
 // ---------------------------------------------------------------------------
-// x and y contractions of one (s, k) plane; out = Tx.v + Ty.v (overwrites)
-__global__ void k_kin_xy_f64(const double* __restrict__ vec, double* __restrict__ out, const double* __restrict__ tx,
-                             const double* __restrict__ ty, int nx, int ny, int nz) {
+// The three contractions of one (s, k) plane, out = Tz.v + (Ty.v + Tx.v).  The plane is in
+// shared memory for x and y; the z columns are read through L2 (coalesced along
+// x, 8 nz bytes per coefficient, a third of the time its nx + ny + nz FP64
+// operations take), so that one launch and no second pass over u_kin remain; T
+// is symmetric and read along its rows by consecutive threads.  13.5 us at 15^3,
+// 21 functions, against 11.4 + 7.4 us for x, y and z in two launches (and one
+// launch less); 27 against 22 + 14 us at 21^3.
+__global__ void k_kin_f64(const double* __restrict__ vec, double* __restrict__ out, const double* __restrict__ tx,
+                          const double* __restrict__ ty, const double* __restrict__ tz, int nx, int ny, int nz) {
   extern __shared__ double plane[];
   const int k = blockIdx.x, s = blockIdx.y;
-  const long long base = ((long long)s * nz + k) * ny * nx;
   const int np = nx * ny;
+  const long long sb = (long long)s * nz * np, base = sb + (long long)k * np;
   for (int e = threadIdx.x; e < np; e += blockDim.x) plane[e] = vec[base + e];
   __syncthreads();
+  const double* tzr = tz + (long long)k * nz;
   for (int e = threadIdx.x; e < np; e += blockDim.x) {
     const int j = e / nx, i = e - j * nx;
-    const double* tr = tx + (long long)i * nx;
+    const double* col = vec + sb + e;
     const double* row = plane + j * nx;
-    double ax = 0.0;
-    for (int q = 0; q < nx; ++q) ax += __ldg(tr + q) * row[q];
-    const double* tc = ty + (long long)j * ny;
-    double ay = 0.0;
-    for (int q = 0; q < ny; ++q) ay += __ldg(tc + q) * plane[q * nx + i];
-    out[base + e] = ay + ax;
-  }
-}
-
-// z contraction of one (s, j) plane, added: out += Tz.v
-__global__ void k_kin_z_f64(const double* __restrict__ vec, double* __restrict__ out, const double* __restrict__ tz,
-                            int nx, int ny, int nz) {
-  extern __shared__ double plane[];  // [k][i]
-  const int j = blockIdx.x, s = blockIdx.y;
-  const long long sb = (long long)s * nz * ny * nx;
-  const int np = nx * nz;
-  for (int e = threadIdx.x; e < np; e += blockDim.x) {
-    const int k = e / nx, i = e - k * nx;
-    plane[e] = vec[sb + ((long long)k * ny + j) * nx + i];
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < np; e += blockDim.x) {
-    const int k = e / nx, i = e - k * nx;
-    const double* tr = tz + (long long)k * nz;
-    double az = 0.0;
-    for (int q = 0; q < nz; ++q) az += __ldg(tr + q) * plane[q * nx + i];
-    const long long o = sb + ((long long)k * ny + j) * nx + i;
-    out[o] = az + out[o];
+    const double* tyr = ty + (long long)j * ny;
+    double ax = 0.0, ay = 0.0, az = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < nz; ++q) az += __ldg(tzr + q) * __ldg(col + (long long)q * np);
+#pragma unroll 4
+    for (int q = 0; q < nx; ++q) ax += __ldg(tx + q * nx + i) * row[q];
+#pragma unroll 4
+    for (int q = 0; q < ny; ++q) ay += __ldg(tyr + q) * plane[q * nx + i];
+    out[base + e] = az + (ay + ax);
   }
 }
 
@@ -511,10 +499,8 @@ __global__ void k_gather_mixed(const double* __restrict__ full, float* __restric
 // r - alpha v = sr (R - alpha (sv/sr) V), beta^2 = sr^2 |R|^2, and the scales of
 // the next iteration, whose V is this R (v_{j+1} = (sr/beta) R) and whose R is
 // this V (r_{j+1} = -beta v_j = (-beta sv) V): no pass rescales or swaps memory.
-// It also writes the FP32 copy of the next v's buffer for the mixed kernels.
 __global__ void k_update_fold(const double* __restrict__ V, double* __restrict__ R, long long L,
-                              float* __restrict__ v32_next, long long D, double* partials, unsigned int* counter,
-                              double* scalars, double* hist, int hist_stride, int j, int* status) {
+                              double* partials, unsigned int* counter, double* scalars, double* hist, int hist_stride, int j, int* status) {
   const double alpha = scalars[0], sv = scalars[4], sr = scalars[5], c = scalars[6];
   const double a = alpha * c;
   double acc = 0.0;
@@ -529,18 +515,11 @@ __global__ void k_update_fold(const double* __restrict__ V, double* __restrict__
     R2[i] = r;
     acc = fma(r.x, r.x, acc);
     acc = fma(r.y, r.y, acc);
-    const long long e = 2 * i;
-    if (e + 1 < D) {
-      reinterpret_cast<float2*>(v32_next)[i] = make_float2(f32_round(r.x), f32_round(r.y));
-    } else if (e < D) {
-      v32_next[e] = f32_round(r.x);
-    }
   }
   if ((L & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
     const double x = fma(-a, V[L - 1], R[L - 1]);
     R[L - 1] = x;
     acc = fma(x, x, acc);
-    if (L - 1 < D) v32_next[L - 1] = f32_round(x);
   }
   double total;
   if (reduce_grid(acc, partials, counter, &total) && threadIdx.x == 0) {
@@ -688,7 +667,6 @@ int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, 
   DeviceState& d = h->d;
   const Tables& t = h->t;
   const long long N = t.npts;
-  const dim3 g(grid_for(N));
   const long long dpk = N * t.nn;
   if (h->precision == BSL_PREC_MIXED) {
     StreamArgs a = vstream_args(h, v, out);
@@ -697,7 +675,7 @@ int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, 
     a.defer = mode == 2 ? h->defer_reductions : 0;
     return launch_vapply_f32(a, t.nn, s);
   }
-  return launch_vapply_f64(d.vb64, g, s, t.nn, v, d.ukin, d.rot, out, N, mode, d.partials, d.counter, d.scalars,
+  return launch_vapply_f64(d.vb64, s, t.nn, v, d.ukin, d.rot, out, N, mode, d.partials, d.counter, d.scalars,
                            d.hist, j, dpk);
 }
 
@@ -713,26 +691,25 @@ int launch_kin_z(bsl_handle* h, const float2* vpair, cudaStream_t s) {
   return h->kinetic_engine == BSL_KIN_TENSOR ? launch_kin_z_tc(h, vpair, s) : launch_kin_z_mixed(h, h->d.v32, s);
 }
 
-int launch_kinetic(bsl_handle* h, const double* v, const float2* vpair, cudaStream_t s) {
+int launch_kin_f64(bsl_handle* h, const double* v, cudaStream_t s) {
   DeviceState& d = h->d;
   const Tables& t = h->t;
-  const bool mixed = h->precision == BSL_PREC_MIXED;
-  const size_t esz = mixed ? sizeof(float) : sizeof(double);
-  const size_t sm_xy = esz * t.nx * t.ny, sm_z = esz * t.nx * t.nz;
-  if (sm_xy > 200 * 1024 || sm_z > 200 * 1024) return fail(BSL_ERR_UNSUPPORTED, "grid plane too large for one CTA");
-  const dim3 gxy(t.nz, t.nn), gz(t.ny, t.nn);
-  if (mixed) {
-    int rc = launch_kin_xy(h, vpair, s);
-    if (!rc) rc = launch_kin_z(h, vpair, s);
-    return rc;
-  } else {
-    cudaFuncSetAttribute(k_kin_xy_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_xy);
-    cudaFuncSetAttribute(k_kin_z_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_z);
-    k_kin_xy_f64<<<gxy, kThreads, sm_xy, s>>>(v, d.ukin, d.tx, d.ty, t.nx, t.ny, t.nz);
-    k_kin_z_f64<<<gz, kThreads, sm_z, s>>>(v, d.ukin, d.tz, t.nx, t.ny, t.nz);
-  }
+  const size_t smem = sizeof(double) * t.nx * t.ny;
+  if (smem > 200 * 1024 || sizeof(double) * t.nx * t.nz > 200 * 1024)
+    return fail(BSL_ERR_UNSUPPORTED, "grid plane too large for one CTA");
+  cudaFuncSetAttribute(k_kin_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int threads = std::min(kThreads, (t.nx * t.ny + 31) / 32 * 32);
+  k_kin_f64<<<dim3(t.nz, t.nn), threads, smem, s>>>(v, d.ukin, d.tx, d.ty, d.tz, t.nx, t.ny, t.nz);
   BSL_CUDA(cudaGetLastError());
   return BSL_OK;
+}
+
+int launch_kinetic(bsl_handle* h, const double* v, const float2* vpair, cudaStream_t s) {
+  if (h->precision == BSL_PREC_MIXED) {
+    const int rc = launch_kin_xy(h, vpair, s);
+    return rc ? rc : launch_kin_z(h, vpair, s);
+  }
+  return launch_kin_f64(h, v, s);
 }
 
 }  // namespace
@@ -1031,7 +1008,7 @@ int launch_update(bsl_handle* h, double* V, double* R, long long L, int j, cudaS
                         reinterpret_cast<float2*>(R), L, h->kinetic_engine == BSL_KIN_TENSOR ? nullptr : d.v32, L - 1,
                         d.partials, d.counter, d.scalars, d.hist, d.hist_cap, j, d.status));
   else
-    k_update_fold<<<d.red_blocks, kThreads, 0, s>>>(V, R, L, d.v32, L - 1, d.partials, d.counter, d.scalars, d.hist,
+    k_update_fold<<<std::min<long long>(d.red_blocks, grid_for(L / 2)), kThreads, 0, s>>>(V, R, L, d.partials, d.counter, d.scalars, d.hist,
                                                     d.hist_cap, j, d.status);
   BSL_CUDA(cudaGetLastError());
   return BSL_OK;
@@ -1068,8 +1045,9 @@ int dev_lanczos_iteration(bsl_handle* h, int j, cudaStream_t s) {
   double* V = h->lanczos_flip ? d.rvec : d.vec;
   double* R = h->lanczos_flip ? d.vec : d.rvec;
   h->defer_reductions = j == 0 && device_counted_iterations(h) ? 1 : 0;
+  const bool fused = h->defer_reductions && fused_iterations(h);
   int rc = launch_kinetic(h, V, reinterpret_cast<const float2*>(V), s);
-  if (h->defer_reductions && fused_iterations(h)) {
+  if (fused) {
     // the block product of V was formed by the previous update (or
     // dev_begin_iterations); this update forms the next one
     StreamArgs a = vstream_args(h, V, R);
@@ -1136,25 +1114,12 @@ int dev_lanczos_iteration_timed(bsl_handle* h, int j, cudaStream_t s, cudaEvent_
   const bool mixed = h->precision == BSL_PREC_MIXED;
   double* V = h->lanczos_flip ? d.rvec : d.vec;
   double* R = h->lanczos_flip ? d.vec : d.rvec;
-  const size_t sm_xy = sizeof(double) * t.nx * t.ny, sm_z = sizeof(double) * t.nx * t.nz;
-  const dim3 gxy(t.nz, t.nn), gz(t.ny, t.nn);
-  if (!mixed) {
-    cudaFuncSetAttribute(k_kin_xy_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_xy);
-    cudaFuncSetAttribute(k_kin_z_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_z);
-  }
+  const float2* Vp = reinterpret_cast<const float2*>(V);
   int rc;
   cudaEventRecord(ev[0], s);
-  if (mixed) {
-    if ((rc = launch_kin_xy(h, reinterpret_cast<const float2*>(V), s))) return rc;
-  } else {
-    k_kin_xy_f64<<<gxy, kThreads, sm_xy, s>>>(V, d.ukin, d.tx, d.ty, t.nx, t.ny, t.nz);
-  }
+  if ((rc = mixed ? launch_kin_xy(h, Vp, s) : launch_kin_f64(h, V, s))) return rc;
   cudaEventRecord(ev[1], s);
-  if (mixed) {
-    if ((rc = launch_kin_z(h, reinterpret_cast<const float2*>(V), s))) return rc;
-  } else {
-    k_kin_z_f64<<<gz, kThreads, sm_z, s>>>(V, d.ukin, d.tz, t.nx, t.ny, t.nz);
-  }
+  if ((rc = mixed ? launch_kin_z(h, Vp, s) : BSL_OK)) return rc;
   cudaEventRecord(ev[2], s);
   const bool fused = h->defer_reductions && fused_iterations(h);
   const StreamArgs fa = vstream_args(h, V, R);
@@ -1170,7 +1135,7 @@ int dev_lanczos_iteration_timed(bsl_handle* h, int j, cudaStream_t s, cudaEvent_
 
 const char* dev_stage_name(bsl_handle* h, int i) {
   const bool mixed = h->precision == BSL_PREC_MIXED;
-  static const char* n64[4] = {"k_kin_xy_f64", "k_kin_z_f64", "k_vapply<NN,double>", "k_update_fold"};
+  static const char* n64[4] = {"k_kin_f64", "(in k_kin_f64)", "k_vapply<NN,double>", "k_update_fold"};
   static const char* nmx[4] = {"k_kin_xy_split", "k_kin_z_split", "k_vstream<NN>", "k_update_pair"};
   static const char* nts[2] = {"k_kin_small", "(in k_kin_small)"};
   static const char* ntc[4] = {"k_kin_xy_tc", "k_kin_z_tc", "k_vstream<NN>", "k_update_stream"};

@@ -831,7 +831,7 @@ int bsl_stage_times(bsl_handle* h, int iters, double* ms, const char** names) {
 
 int bsl_launches_per_iteration(const bsl_handle* h) {
   if (!h) return -1;
-  const bool one = h->precision == BSL_PREC_MIXED && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h);
+  const bool one = h->precision != BSL_PREC_MIXED || (h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h));
   return one ? 3 : 4;  // kinetic in one launch or two
 }
 

@@ -12,8 +12,9 @@ namespace {
 //   mode 0: u = T v + rot v + V v          (u = out)
 //   mode 1: r += T v + rot v + V v; partial alpha = v . r   (r = out, in place)
 // ---------------------------------------------------------------------------
+constexpr int kVapplyThreads = kThreads;
 template <int NN, typename VT>
-__global__ void __launch_bounds__(kThreads) k_vapply(const VT* __restrict__ vb, const double* __restrict__ vec,
+__global__ void __launch_bounds__(kVapplyThreads) k_vapply(const VT* __restrict__ vb, const double* __restrict__ vec,
                                                      const double* __restrict__ ukin, const double* __restrict__ rot,
                                                      double* __restrict__ out, long long npts, int mode,
                                                      double* partials, unsigned int* counter, double* scalars,
@@ -57,6 +58,67 @@ __global__ void __launch_bounds__(kThreads) k_vapply(const VT* __restrict__ vb, 
   }
   if (mode == 1) {
     if (p == 0) dot += vec[dpk] * out[dpk];  // the coordinate outside the symmetry block (H acts on it as 0)
+    double total;
+    if (reduce_grid(dot, partials, counter, &total) && threadIdx.x == 0) {
+      scalars[0] = scalars[7] * total;
+      hist[j - 1] = scalars[7] * total;
+    }
+  }
+}
+
+// The same for grids whose points are too few warps to fill the FP64 pipes:
+// a CTA takes 32 points, and each of its kG warps NN / kG rows of their blocks.
+// A row's sum runs over the columns in the order in which k_vapply adds them,
+// so H v is the same bits.
+template <int NN, int kG>
+__global__ void __launch_bounds__(32 * kG) k_vapply_rows(const double* __restrict__ vb,
+                                                         const double* __restrict__ vec,
+                                                         const double* __restrict__ ukin,
+                                                         const double* __restrict__ rot, double* __restrict__ out,
+                                                         long long npts, int mode, double* partials,
+                                                         unsigned int* counter, double* scalars, double* hist, int j,
+                                                         long long dpk) {
+  constexpr int R = NN / kG;
+  static_assert(R * kG == NN, "the rows are split evenly");
+  const int s0 = (threadIdx.x >> 5) * R;
+  const long long p = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
+  const double c = mode ? scalars[6] : 1.0;
+  double dot = 0.0;
+  if (p < npts) {
+    double v[NN], va[R], acc[R], vr[R];
+#pragma unroll
+    for (int q = 0; q < NN; ++q) v[q] = vec[q * npts + p];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int s = s0 + r;
+      va[r] = 0.0;
+      vr[r] = vec[s * npts + p];
+      acc[r] = ukin[s * npts + p] + __ldg(rot + s) * vr[r];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int s = s0 + r;
+#pragma unroll
+      for (int q = 0; q < NN; ++q) {
+        const int a = q < s ? q : s, b = q < s ? s : q;  // element (a, b), a <= b, of the triangle
+        va[r] += vb[(long long)(a * NN - a * (a - 1) / 2 + b - a) * npts + p] * v[q];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const long long i = (s0 + r) * npts + p;
+      const double hv = acc[r] + va[r];
+      if (mode == 0) {
+        out[i] = hv;
+      } else {
+        const double x = fma(c, hv, out[i]);
+        out[i] = x;
+        dot += vr[r] * x;
+      }
+    }
+  }
+  if (mode == 1) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) dot += vec[dpk] * out[dpk];
     double total;
     if (reduce_grid(dot, partials, counter, &total) && threadIdx.x == 0) {
       scalars[0] = scalars[7] * total;

@@ -1,15 +1,15 @@
-"""The size-dependent kernels of H v and of the Lanczos iteration against one
-another, at the edges of their ranges.
+"""The size-dependent kernels of H v and of the Lanczos iteration against the
+oracle and against one another, at the edges of their ranges.
 
-Mixed: the kinetic in one launch up to 16 points per axis, the same bits as the
-tensor-core kernels'.
+FP64: the block product split over rows up to 26,000 points.  Mixed: the kinetic in one launch
+up to 16 points per axis, the same bits as the tensor-core kernels'.
 """
 import os
 
 import numpy as np
 import pytest
 
-from conftest import load_inputs, load_package
+from conftest import OracleModel, load_inputs, load_package
 
 pytestmark = pytest.mark.gpu
 CALC = "linRotCartSph_NoQuad_ContGrid_Alavi_SPCE"
@@ -32,8 +32,55 @@ def write_case(tmp, n, l_max, sym):
     return hv
 
 
+# 26,000 points from below and above, a last warp of one point, blocks with and
+# without the row split, planes of unequal edges
+@pytest.mark.parametrize("n,l_max,sym", [
+    ((23, 23, 23), 4, "Even"), ((25, 25, 23), 5, "Odd"), ((17, 17, 64), 5, "All"), ((33, 33, 25), 3, "Odd"),
+    ((64, 64, 7), 5, "Odd"), ((29, 29, 31), 3, "All"), ((13, 11, 9), 2, "All"), ((32, 31, 26), 4, "Even"),
+    ((5, 5, 13), 6, "Even"), ((48, 48, 20), 1, "All")])
+def test_fp64_hv(bsl, tmp_path, n, l_max, sym):
+    hv = write_case(str(tmp_path), n, l_max, sym)
+    h = bsl.Hamiltonian(hv, CALC, precision="fp64")
+    m = OracleModel(CALC, hv, threads=os.cpu_count() or 8)
+    try:
+        rng = np.random.default_rng(3)
+        z = np.linspace(-3, 3, n[2])[:, None, None] ** 2 + np.linspace(-3, 3, n[1])[:, None] ** 2 + np.linspace(
+            -3, 3, n[0]) ** 2
+        for v in (rng.standard_normal(h.basis_size), np.tile(np.exp(-z).ravel(), h.basis_size // z.size),
+                  1e-200 * rng.standard_normal(h.basis_size)):
+            u = np.zeros_like(v)
+            h.hv(v, u)
+            ref = m.hv(v)
+            # a dot product of nx + ny + nz + nn terms, each rounded at 2^-53 of the
+            # largest partial sum (max |T| max |v|, up to 3 x its result's size here)
+            tol = 2.0 ** -53 * sum(n) * 3
+            scale = np.max(np.abs(v)) * max(np.max(np.abs(ref)) / np.max(np.abs(v)), kinetic_scale(n))
+            assert np.max(np.abs(u - ref)) <= tol * scale
+    finally:
+        h.close()
+        m.close()
+
+
 def kinetic_scale(n):
     return sum(0.0635077857002 ** 2 / (2 * 2.01588) * np.pi ** 2 / 3 * ((k - 1) / 0.08) ** 2 for k in n)
+
+
+def test_fp64_hv_of_non_finite_and_zero_vectors(bsl, tmp_path):
+    """An infinity or a NaN reaches every line through its point, a zero vector stays zero."""
+    h = bsl.Hamiltonian(write_case(str(tmp_path), (26, 26, 26), 5, "Odd"), CALC, precision="fp64")
+    try:
+        u = np.zeros(h.basis_size)
+        h.hv(np.zeros(h.basis_size), u)
+        assert np.all(u == 0.0)
+        for bad in (np.inf, np.nan):
+            v = np.ones(h.basis_size)
+            v[26 * 26 * 11 + 26 * 7 + 5] = bad  # function 0 is l = 5, m = -5
+            u = np.zeros(h.basis_size)
+            h.hv(v, u)
+            w = u[:26 ** 3].reshape(26, 26, 26)
+            assert not np.any(np.isfinite(np.concatenate([w[11, 7], w[11, :, 5], w[:, 7, 5]])))
+    finally:
+        h.close()
 
 
 # one launch up to 16 points: smallest grids, planes of a full and of a broken warp
