@@ -332,6 +332,8 @@ void free_device(DeviceState& d) {
   if (d.kz_slices) cudaFree(d.kz_slices);
   if (d.tx_slices32) cudaFree(d.tx_slices32);
   if (d.tz_slices32) cudaFree(d.tz_slices32);
+  if (d.kxy_slices64) cudaFree(d.kxy_slices64);
+  if (d.kz_slices64) cudaFree(d.kz_slices64);
   if (d.jdev) cudaFree(d.jdev);
   if (d.vb16) cudaFree(d.vb16);
   if (d.vscale) cudaFree(d.vscale);
@@ -441,6 +443,10 @@ int hv_prep(const bsl_hv_params* params, const Cage* cage, bsl_handle** out) {
     if ((rc = upload(&d.tx_slices32, sf, "Tx"))) return bail(rc);
     kinetic_slices_f32(t.tz, t.nz, &sf);
     if ((rc = upload(&d.tz_slices32, sf, "Tz"))) return bail(rc);
+    kinetic_smem_image64(t.tx, t.nx, true, &sl, &d.e_txy64);
+    if ((rc = upload(&d.kxy_slices64, sl, "Tx"))) return bail(rc);
+    kinetic_smem_image64(t.tz, t.nz, false, &sl, &d.e_tz64);
+    if ((rc = upload(&d.kz_slices64, sl, "Tz"))) return bail(rc);
     h->kinetic_engine = BSL_KIN_TENSOR;
   }
   if ((rc = upload(&d.rot, t.rot, "rotor"))) return bail(rc);

@@ -100,6 +100,9 @@ struct DeviceState {
   uint16_t *kxy_slices = nullptr, *kz_slices = nullptr;
   int e_txy = 0, e_tz = 0;
   float *tx_slices32 = nullptr, *tz_slices32 = nullptr;  // the slices as FP32 integers (bsl_small.cu)
+  // the same for the FP64 path: seven slices (bsl_kinetic_tc64.cu)
+  uint16_t *kxy_slices64 = nullptr, *kz_slices64 = nullptr;
+  int e_txy64 = 0, e_tz64 = 0;
   int kin_grid_xy = 0, kin_grid_z = 0;  // persistent grid sizes
   double* rot = nullptr;  // [nn]
   // potential grid V(p, a, b) for phi_b and 2pi - phi_b, p in vector order
@@ -231,6 +234,11 @@ void kinetic_slices_f32(const std::vector<double>& T, int n, std::vector<float>*
 // block totals of a deferred beta to finish
 bool kin_small_supported(const bsl_handle* h);
 int launch_kin_small(bsl_handle* h, const float2* v, int fin_count, cudaStream_t s);
+// FP64 kinetic on the tensor cores (bsl_kinetic_tc64.cu): FP64 v, FP64 output
+void kinetic_smem_image64(const std::vector<double>& T, int n, bool with_zero_tiles, std::vector<uint16_t>* image,
+                          int* e_t);
+int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s);
+bool kin_f64_tensor(const bsl_handle* h);
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 int launch_kin_z_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 // grouped tensor-core kinetic over several problems: per-problem argument

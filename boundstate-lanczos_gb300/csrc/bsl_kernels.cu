@@ -369,7 +369,8 @@ __global__ void k_vblocks(BlockTables bt, const double* v1, const double* v2, lo
 // ---------------------------------------------------------------------------
 // kinetic
 // ---------------------------------------------------------------------------
-// The three contractions of one (s, k) plane, out = Tz.v + (Ty.v + Tx.v).  The plane is in
+// The three contractions of one (s, k) plane, out = Tz.v + (Ty.v + Tx.v), for the
+// grids that do not run on the tensor cores (launch_kinetic).  The plane is in
 // shared memory for x and y; the z columns are read through L2 (coalesced along
 // x, 8 nz bytes per coefficient, a third of the time its nx + ny + nz FP64
 // operations take), so that one launch and no second pass over u_kin remain; T
@@ -691,7 +692,11 @@ int launch_kin_z(bsl_handle* h, const float2* vpair, cudaStream_t s) {
   return h->kinetic_engine == BSL_KIN_TENSOR ? launch_kin_z_tc(h, vpair, s) : launch_kin_z_mixed(h, h->d.v32, s);
 }
 
-int launch_kin_f64(bsl_handle* h, const double* v, cudaStream_t s) {
+// FP64 kinetic stage: x and y (xy) into d.ukin, or z added to it; without the
+// tensor cores all three in the first stage and nothing in the second
+int launch_kin_f64(bsl_handle* h, const double* v, bool xy, cudaStream_t s) {
+  if (kin_f64_tensor(h)) return launch_kin_tc64(h, v, xy, s);
+  if (!xy) return BSL_OK;
   DeviceState& d = h->d;
   const Tables& t = h->t;
   const size_t smem = sizeof(double) * t.nx * t.ny;
@@ -705,14 +710,22 @@ int launch_kin_f64(bsl_handle* h, const double* v, cudaStream_t s) {
 }
 
 int launch_kinetic(bsl_handle* h, const double* v, const float2* vpair, cudaStream_t s) {
-  if (h->precision == BSL_PREC_MIXED) {
-    const int rc = launch_kin_xy(h, vpair, s);
-    return rc ? rc : launch_kin_z(h, vpair, s);
-  }
-  return launch_kin_f64(h, v, s);
+  int rc;
+  if (h->precision == BSL_PREC_MIXED)
+    return (rc = launch_kin_xy(h, vpair, s)) ? rc : launch_kin_z(h, vpair, s);
+  return (rc = launch_kin_f64(h, v, true, s)) ? rc : launch_kin_f64(h, v, false, s);
 }
 
 }  // namespace
+
+// Whether the FP64 kinetic runs on the tensor cores: from 1.6e7 multiply-adds
+// on, which take the FP64 pipes as long (25 us) as the tensor-core kernels' set-up
+// and one plane pair per SM.  Measured, both contractions, odd l <= 5: 39 against 49
+// us at 21^3 (1.2e7), 62 against 52 us at 24^3 (2.1e7), 993 against 127 us at 54^3.
+bool kin_f64_tensor(const bsl_handle* h) {
+  const Tables& t = h->t;
+  return h->d.kxy_slices64 && (double)t.npts * t.nn * (t.nx + t.ny + t.nz) >= 1.6e7;
+}
 
 // ---------------------------------------------------------------------------
 // launchers
@@ -1117,9 +1130,9 @@ int dev_lanczos_iteration_timed(bsl_handle* h, int j, cudaStream_t s, cudaEvent_
   const float2* Vp = reinterpret_cast<const float2*>(V);
   int rc;
   cudaEventRecord(ev[0], s);
-  if ((rc = mixed ? launch_kin_xy(h, Vp, s) : launch_kin_f64(h, V, s))) return rc;
+  if ((rc = mixed ? launch_kin_xy(h, Vp, s) : launch_kin_f64(h, V, true, s))) return rc;
   cudaEventRecord(ev[1], s);
-  if ((rc = mixed ? launch_kin_z(h, Vp, s) : BSL_OK)) return rc;
+  if ((rc = mixed ? launch_kin_z(h, Vp, s) : launch_kin_f64(h, V, false, s))) return rc;
   cudaEventRecord(ev[2], s);
   const bool fused = h->defer_reductions && fused_iterations(h);
   const StreamArgs fa = vstream_args(h, V, R);
@@ -1136,10 +1149,11 @@ int dev_lanczos_iteration_timed(bsl_handle* h, int j, cudaStream_t s, cudaEvent_
 const char* dev_stage_name(bsl_handle* h, int i) {
   const bool mixed = h->precision == BSL_PREC_MIXED;
   static const char* n64[4] = {"k_kin_f64", "(in k_kin_f64)", "k_vapply<NN,double>", "k_update_fold"};
+  static const char* n64t[2] = {"k_kin_xy_tc64", "k_kin_z_tc64"};
   static const char* nmx[4] = {"k_kin_xy_split", "k_kin_z_split", "k_vstream<NN>", "k_update_pair"};
   static const char* nts[2] = {"k_kin_small", "(in k_kin_small)"};
   static const char* ntc[4] = {"k_kin_xy_tc", "k_kin_z_tc", "k_vstream<NN>", "k_update_stream"};
-  if (!mixed) return n64[i];
+  if (!mixed) return i < 2 && kin_f64_tensor(h) ? n64t[i] : n64[i];
   if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)) return nts[i];
   if (fused_iterations(h) && i >= 2)
     return i == 2 ? "k_vapply_light<NN>" : h->vformat == BSL_VFMT_GAUNT ? "k_vstream<NN,coefficients,update>"

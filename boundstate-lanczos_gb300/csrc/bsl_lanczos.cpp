@@ -831,8 +831,10 @@ int bsl_stage_times(bsl_handle* h, int iters, double* ms, const char** names) {
 
 int bsl_launches_per_iteration(const bsl_handle* h) {
   if (!h) return -1;
-  const bool one = h->precision != BSL_PREC_MIXED || (h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h));
-  return one ? 3 : 4;  // kinetic in one launch or two
+  // kinetic in one launch: small grids in mixed precision, FP64 without the tensor cores
+  const bool one = h->precision == BSL_PREC_MIXED ? h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)
+                                                  : !kin_f64_tensor(h);
+  return one ? 3 : 4;
 }
 
 int bsl_debug_inject_timeout(bsl_handle* h, int kernel_mask) {

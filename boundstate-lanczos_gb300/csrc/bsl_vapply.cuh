@@ -12,9 +12,14 @@ namespace {
 //   mode 0: u = T v + rot v + V v          (u = out)
 //   mode 1: r += T v + rot v + V v; partial alpha = v . r   (r = out, in place)
 // ---------------------------------------------------------------------------
-constexpr int kVapplyThreads = kThreads;
+// The FP64 apply is bound by the FP64 pipe (nn^2 + 4 nn operations a point at
+// 2 lanes a clock and SM: 131 us at 54^3 and 21 functions).  Blocks of 128 points
+// at 4 per SM, so that an SM holds warps in different phases and no last wave of
+// large blocks idles: 187 us there against 229 us with blocks of 256 points (4.05
+// waves of one block per SM), 86 against 98 us at 41^3.
+constexpr int kVapplyThreads = 128;
 template <int NN, typename VT>
-__global__ void __launch_bounds__(kVapplyThreads) k_vapply(const VT* __restrict__ vb, const double* __restrict__ vec,
+__global__ void __launch_bounds__(kVapplyThreads, NN <= 21 ? 4 : 1) k_vapply(const VT* __restrict__ vb, const double* __restrict__ vec,
                                                      const double* __restrict__ ukin, const double* __restrict__ rot,
                                                      double* __restrict__ out, long long npts, int mode,
                                                      double* partials, unsigned int* counter, double* scalars,

@@ -1,7 +1,8 @@
 """The size-dependent kernels of H v and of the Lanczos iteration against the
 oracle and against one another, at the edges of their ranges.
 
-FP64: the block product split over rows up to 26,000 points.  Mixed: the kinetic in one launch
+FP64: the kinetic on the tensor cores from 1.6e7 multiply-adds on, the block
+product split over rows up to 26,000 points.  Mixed: the kinetic in one launch
 up to 16 points per axis, the same bits as the tensor-core kernels'.
 """
 import os
@@ -32,8 +33,10 @@ def write_case(tmp, n, l_max, sym):
     return hv
 
 
-# 26,000 points from below and above, a last warp of one point, blocks with and
-# without the row split, planes of unequal edges
+# kinetic: plain just below 1.6e7 (23^3 at 15 functions), tensor cores above it, an
+# odd number of planes, a last pair of one plane, 16-row steps with 1 and 16 rows,
+# 64 points; block product: 26,000 points from below and above, a last warp of
+# one point, blocks with and without the row split
 @pytest.mark.parametrize("n,l_max,sym", [
     ((23, 23, 23), 4, "Even"), ((25, 25, 23), 5, "Odd"), ((17, 17, 64), 5, "All"), ((33, 33, 25), 3, "Odd"),
     ((64, 64, 7), 5, "Odd"), ((29, 29, 31), 3, "All"), ((13, 11, 9), 2, "All"), ((32, 31, 26), 4, "Even"),
