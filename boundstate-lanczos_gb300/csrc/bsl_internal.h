@@ -255,7 +255,8 @@ int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nct
 // FP32 blocks in the tile-major layout of bsl_vstream.cu (vstream_tile_points() points per tile)
 struct StreamArgs {
   const float* vb;      // tile-major FP32 blocks
-  const float* v32;     // FP32 copy of v
+  const float* v32;     // FP32 copy of v (mode 0 and 1 of the CUDA-core kinetic)
+  const float2* vpair;  // mode 0 of the tensor-core kinetic: v as pairs, whose heads take its place
   const double* vec;    // FP64 v (alpha dot product, extra coordinate)
   const float2* ukin;   // kinetic (hi, lo) pairs
   const float* rot_hi;  // rotor energies, head and tail

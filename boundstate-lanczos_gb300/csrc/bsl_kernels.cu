@@ -491,7 +491,7 @@ __global__ void k_gather_mixed(const double* __restrict__ full, float* __restric
   const long long p = e - (long long)s * npts;
   const double x = full[(long long)full_of[s] * npts + p];
   const float2 d = df_of(x);
-  v32[e] = d.x;
+  if (v32) v32[e] = d.x;  // the CUDA-core kinetic's operand
   if (vpair) vpair[e] = d;
 }
 
@@ -671,6 +671,7 @@ int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, 
   const long long dpk = N * t.nn;
   if (h->precision == BSL_PREC_MIXED) {
     StreamArgs a = vstream_args(h, v, out);
+    a.vpair = mode == 0 && h->kinetic_engine == BSL_KIN_TENSOR ? d.vpair : nullptr;
     a.mode = mode;
     a.j = j;
     a.defer = mode == 2 ? h->defer_reductions : 0;
@@ -997,10 +998,11 @@ int dev_hv(bsl_handle* h, const double* v, double* u, cudaStream_t s) {
   DeviceState& d = h->d;
   const long long D = bsl_packed_size(h);
   if (h->precision == BSL_PREC_MIXED) {
-    k_to_f32<<<1024, kThreads, 0, s>>>(v, d.v32, D);
-    if (h->kinetic_engine == BSL_KIN_TENSOR) {
+    if (h->kinetic_engine == BSL_KIN_TENSOR) {  // the heads of the pairs are the FP32 copy
       if (!d.vpair) BSL_CUDA(cudaMalloc(&d.vpair, (size_t)D * sizeof(float2)));
       k_pair_copy<<<1024, kThreads, 0, s>>>(v, d.vpair, D);
+    } else {
+      k_to_f32<<<1024, kThreads, 0, s>>>(v, d.v32, D);
     }
     BSL_CUDA(cudaGetLastError());
   }
@@ -1207,7 +1209,8 @@ int dev_hv_full(bsl_handle* h, const double* full, double* out, cudaStream_t s) 
   }
   const bool tc = h->kinetic_engine == BSL_KIN_TENSOR;
   if (tc && !d.vpair) BSL_CUDA(cudaMalloc(&d.vpair, (size_t)D * sizeof(float2)));
-  k_gather_mixed<<<grid_for(D), kThreads, 0, s>>>(full, d.v32, tc ? d.vpair : nullptr, d.full_of, N, h->t.nn);
+  k_gather_mixed<<<grid_for(D), kThreads, 0, s>>>(full, tc ? nullptr : d.v32, tc ? d.vpair : nullptr, d.full_of, N,
+                                                  h->t.nn);
   BSL_CUDA(cudaGetLastError());
   int rc = launch_kinetic(h, nullptr, d.vpair, s);
   if (rc) return rc;

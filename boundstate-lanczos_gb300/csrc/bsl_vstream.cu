@@ -244,7 +244,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
         vv[s] = x.x;
         vlo[s] = x.y;
       } else {
-        vv[s] = valid ? A.v32[s * npts + p] : 0.f;
+        vv[s] = !valid ? 0.f : A.vpair ? A.vpair[s * npts + p].x : A.v32[s * npts + p];
         vlo[s] = 0.f;
       }
       va[s] = 0.f;
