@@ -212,9 +212,14 @@ int dev_hv_full(bsl_handle* h, const double* full, double* out, cudaStream_t s);
 int dev_full_step_fused(bsl_handle* h, double* v, double* r, long long L, const double* hv, int j, cudaStream_t s,
                         double* v_out = nullptr, double* r_out = nullptr);
 int dev_scatter_full(bsl_handle* h, const double* packed, double* full_accum, cudaStream_t s);
-// previous: the v of the iteration just launched (the buffer roles have flipped)
-int dev_ritz_accumulate(bsl_handle* h, const double* coef, const int* active, int ngood, double* ritz,
-                        cudaStream_t s, bool previous);
+// Ritz accumulation in blocks of ritz_block() iterations: V_j and its scale saved
+// (previous: the v of the iteration just launched, the buffer roles have
+// flipped), then nj of them added to the vectors
+int ritz_block();
+int dev_ritz_save(bsl_handle* h, double* saved, double* sv, cudaStream_t s, bool previous);
+int dev_ritz_accumulate(bsl_handle* h, const double* saved, const double* sv, int nj, const double* coef,
+                        const int* active, int ngood, double* ritz, cudaStream_t s);
+int dev_ritz_full(bsl_handle* h, const double* ritz, int ngood, double off, double* out, cudaStream_t s);
 
 // mixed-precision kinetic (bsl_kinetic.cu)
 void kinetic_split_tables(const std::vector<double>& T, int n, bool transpose, std::vector<float>* head,

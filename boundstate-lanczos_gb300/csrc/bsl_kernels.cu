@@ -652,16 +652,54 @@ __global__ void k_scatter_add(const double* __restrict__ packed, double* __restr
   full[o] = full[o] + packed[e];
 }
 
-// ritz[n*D + i] += coef[n] * v[i] for active n, v = scalars[4] * V
-__global__ void k_ritz(const double* __restrict__ V, long long D, const double* __restrict__ coef,
-                       const int* __restrict__ active, int ngood, double* __restrict__ ritz,
-                       const double* __restrict__ scalars, int pairs) {
-  const double sv = scalars[4];
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (long long)gridDim.x * blockDim.x) {
-    const double vi = sv * (pairs ? f64_of_df(reinterpret_cast<const float2*>(V)[i]) : V[i]);
-    for (int n = 0; n < ngood; ++n)
-      if (active[n]) ritz[(long long)n * D + i] += coef[n] * vi;
+// The Ritz accumulation ritz[n][i] += coef_j[n] v_j[i] for active n, v_j = sv_j V_j,
+// taken kRitzBlock iterations at a time: reading and writing the ngood vectors is
+// the cost (16 ngood bytes a coefficient, 530 MB at 54^3 and 10 levels, as much
+// time as the iteration itself), so the V_j are kept (k_ritz_save, 16 bytes a
+// coefficient) and the vectors pass through once per block.  The terms are added
+// in the order of j, the same bits as one pass per iteration.  bsl_ritz_vectors of
+// 32 iterations and 10 levels at 27^3: 7.5 -> 4.9 ms with the reference layout put
+// together on the device (k_ritz_full) instead of on the host.
+constexpr int kRitzBlock = 8;
+__global__ void k_ritz_save(const double* __restrict__ V, long long L, const double* __restrict__ scalars,
+                            double* __restrict__ saved, double* __restrict__ sv) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < L; i += (long long)gridDim.x * blockDim.x)
+    saved[i] = V[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sv = scalars[4];
+}
+
+__global__ void k_ritz(const double* __restrict__ saved, const double* __restrict__ sv, int nj, long long L,
+                       const double* __restrict__ coef, const int* __restrict__ active, int ngood,
+                       double* __restrict__ ritz, int pairs) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < L; i += (long long)gridDim.x * blockDim.x) {
+    double v[kRitzBlock];
+#pragma unroll
+    for (int j = 0; j < kRitzBlock; ++j)
+      if (j < nj) {
+        const double x = saved[(long long)j * L + i];
+        v[j] = __ldg(sv + j) * (pairs ? f64_of_df(make_float2(__int_as_float(__double2loint(x)), __int_as_float(__double2hiint(x)))) : x);
+      }
+    for (int n = 0; n < ngood; ++n) {
+      double r = ritz[(long long)n * L + i];
+#pragma unroll
+      for (int j = 0; j < kRitzBlock; ++j)
+        if (j < nj && __ldg(active + j * ngood + n)) r += __ldg(coef + j * ngood + n) * v[j];
+      ritz[(long long)n * L + i] = r;
+    }
   }
+}
+
+// the accumulated vectors in the reference layout: packed function s at its full
+// index, the components outside the block from the extra coordinate
+__global__ void k_ritz_full(const double* __restrict__ ritz, const int* __restrict__ packed_of, long long npts, int nn,
+                            int nfull, double off, double* __restrict__ out) {
+  const int f = blockIdx.y, n = blockIdx.z, s = packed_of[f];
+  const long long L = npts * nn + 1;
+  const double* in = ritz + n * L + (s >= 0 ? s * npts : 0);
+  const double masked = ritz[n * L + npts * nn] * off;
+  double* o = out + ((long long)n * nfull + f) * npts;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npts; p += (long long)gridDim.x * blockDim.x)
+    o[p] = s >= 0 ? in[p] : masked;
 }
 
 int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, cudaStream_t s) {
@@ -1233,12 +1271,34 @@ int dev_full_step_fused(bsl_handle* h, double* v, double* r, long long L, const 
   return BSL_OK;
 }
 
-int dev_ritz_accumulate(bsl_handle* h, const double* coef, const int* active, int ngood, double* ritz,
-                        cudaStream_t s, bool previous) {
+int ritz_block() { return kRitzBlock; }
+
+int dev_ritz_save(bsl_handle* h, double* saved, double* sv, cudaStream_t s, bool previous) {
   const long long L = bsl_packed_size(h) + 1;  // with the coordinate outside the symmetry block
   const double* V = (h->lanczos_flip ^ (previous ? 1 : 0)) ? h->d.rvec : h->d.vec;
-  k_ritz<<<1024, kThreads, 0, s>>>(V, L, coef, active, ngood, ritz, h->d.scalars, h->state_pairs == 1);
+  k_ritz_save<<<1024, kThreads, 0, s>>>(V, L, h->d.scalars, saved, sv);
   BSL_CUDA(cudaGetLastError());
+  return BSL_OK;
+}
+
+int dev_ritz_accumulate(bsl_handle* h, const double* saved, const double* sv, int nj, const double* coef,
+                        const int* active, int ngood, double* ritz, cudaStream_t s) {
+  const long long L = bsl_packed_size(h) + 1;
+  k_ritz<<<std::min(grid_for(L), 1 << 16), kThreads, 0, s>>>(saved, sv, nj, L, coef, active, ngood, ritz,
+                                                             h->state_pairs == 1);
+  BSL_CUDA(cudaGetLastError());
+  return BSL_OK;
+}
+
+int dev_ritz_full(bsl_handle* h, const double* ritz, int ngood, double off, double* out, cudaStream_t s) {
+  const Tables& t = h->t;
+  for (int n0 = 0; n0 < ngood; n0 += 65535) {  // grid limit
+    const int n = std::min(ngood - n0, 65535);
+    k_ritz_full<<<dim3((unsigned)std::min(grid_for(t.npts), 1 << 10), t.nn_full, n), kThreads, 0, s>>>(
+        ritz + (long long)n0 * (t.npts * t.nn + 1), h->d.packed_of, t.npts, t.nn, t.nn_full, off,
+        out + (long long)n0 * t.nn_full * t.npts);
+    BSL_CUDA(cudaGetLastError());
+  }
   return BSL_OK;
 }
 

@@ -718,12 +718,17 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
     }
   double* dcoef = nullptr;
   int* dact = nullptr;
-  double* dritz = nullptr;
+  double *dritz = nullptr, *dsaved = nullptr;
+  double* dfull = nullptr;  // the vectors in the reference layout, as many as the device has room for
   auto cleanup = [&]() {
     cudaFree(dcoef);
     cudaFree(dact);
     cudaFree(dritz);
+    cudaFree(dsaved);
+    cudaFree(dfull);
   };
+  // V_j of a block of iterations and their scales; one at a time where memory is short
+  int block = ritz_block();
   cudaError_t e;
   if ((e = cudaMalloc(&dcoef, coef.size() * sizeof(double))) != cudaSuccess ||
       (e = cudaMalloc(&dact, active.size() * sizeof(int))) != cudaSuccess ||
@@ -731,6 +736,16 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
     cleanup();
     return fail(BSL_ERR_NOMEM, std::string("Ritz buffers: ") + cudaGetErrorString(e));
   }
+  while ((e = cudaMalloc(&dsaved, block * ((size_t)L + 1) * sizeof(double))) != cudaSuccess) {
+    cudaGetLastError();
+    dsaved = nullptr;
+    if (block == 1) {
+      cleanup();
+      return fail(BSL_ERR_NOMEM, std::string("Ritz buffers: ") + cudaGetErrorString(e));
+    }
+    block = 1;
+  }
+  double* dsv = dsaved + (size_t)block * L;
   cudaStream_t s = d.stream;
   cudaMemcpyAsync(dcoef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dact, active.data(), active.size() * sizeof(int), cudaMemcpyHostToDevice, s);
@@ -746,41 +761,41 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
     cleanup();
     return rc;
   }
-  for (int j = 1; j <= niter; ++j) {
-    const double* cj = dcoef + (size_t)(j - 1) * ngood;
-    const int* aj = dact + (size_t)(j - 1) * ngood;
-    if (counted) {
-      rc = dev_lanczos_iteration(h, 0, s);
-      if (!rc) rc = dev_ritz_accumulate(h, cj, aj, ngood, dritz, s, true);
-    } else {
-      rc = dev_ritz_accumulate(h, cj, aj, ngood, dritz, s, false);
-      if (!rc) rc = dev_lanczos_iteration(h, j, s);
-    }
-    if (rc) {
-      cleanup();
-      return rc;
+  int nj = 0;  // V_j saved since the last accumulation
+  for (int j = 1; j <= niter && !rc; ++j) {
+    if (counted) rc = dev_lanczos_iteration(h, 0, s);
+    if (!rc) rc = dev_ritz_save(h, dsaved + (size_t)nj * L, dsv + nj, s, counted);
+    if (!rc && !counted) rc = dev_lanczos_iteration(h, j, s);
+    if (!rc && (++nj == block || j == niter)) {
+      const size_t c0 = (size_t)(j - nj) * ngood;
+      rc = dev_ritz_accumulate(h, dsaved, dsv, nj, dcoef + c0, dact + c0, ngood, dritz, s);
+      nj = 0;
     }
   }
-  if (counted && (rc = dev_finish_iterations(h, s))) {
-    cleanup();
-    return rc;
+  if (!rc && counted) rc = dev_finish_iterations(h, s);
+  // the reference layout is put together on the device and copied straight into
+  // the caller's buffer, a few vectors at a time where memory is short
+  cudaFree(dsaved);
+  dsaved = nullptr;
+  int group = ngood;
+  while (!rc && cudaMalloc(&dfull, (size_t)group * Df * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    dfull = nullptr;
+    if (group == 1) rc = fail(BSL_ERR_NOMEM, "Ritz vectors");
+    group = (group + 1) / 2;
   }
-  std::vector<double> host((size_t)ngood * L);
-  e = cudaMemcpyAsync(host.data(), dritz, host.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cleanup();
-  if (e != cudaSuccess) return cuda_fail(e, "Ritz vectors");
-  const Tables& t = h->t;
-  const long long N = t.npts;
   const double off = (Df > D) ? 1.0 / std::sqrt((double)(Df - D)) : 0.0;
-  for (int n = 0; n < ngood; ++n) {
-    double* out = ritz + (size_t)n * Df;
-    const double* in = host.data() + (size_t)n * L;
-    const double masked = in[D] * off;
-    for (long long i = 0; i < Df; ++i) out[i] = masked;
-    for (int sidx = 0; sidx < t.nn; ++sidx)
-      std::memcpy(out + (size_t)t.full_of[sidx] * N, in + (size_t)sidx * N, N * sizeof(double));
+  for (int n0 = 0; n0 < ngood && !rc; n0 += group) {
+    const int n = std::min(group, ngood - n0);
+    if ((rc = dev_ritz_full(h, dritz + (size_t)n0 * L, n, off, dfull, s))) break;
+    if ((e = cudaMemcpyAsync(ritz + (size_t)n0 * Df, dfull, (size_t)n * Df * sizeof(double), cudaMemcpyDeviceToHost,
+                             s)) != cudaSuccess)
+      rc = cuda_fail(e, "Ritz vectors");
   }
+  e = cudaStreamSynchronize(s);
+  cleanup();
+  if (rc) return rc;
+  if (e != cudaSuccess) return cuda_fail(e, "Ritz vectors");
   return check_status(h);
 }
 
