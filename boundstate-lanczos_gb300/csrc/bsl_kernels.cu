@@ -173,14 +173,35 @@ __global__ void k_potential_coulomb(const double* xg, const double* yg, const do
   v2[t] = v;
 }
 
-// RN(k / RN(sqrt(r2))), the two correctly rounded FP64 operations, in 6 FP64
+// The double h + l for h a normal float and |l| a few ulps of h, from the integer
+// pipe: the mantissa of h plus l as a fixed-point number of units 2^-50 of h's
+// binade (l rounded to those units).
+__device__ __forceinline__ double double_of(float h, float l) {
+  const unsigned int hb = __float_as_uint(h) & 0x7FFFFFFFu, ex = hb >> 23;
+  const int n = __float2int_rn(__fmul_rn(__uint_as_float(__float_as_uint(l) ^ (__float_as_uint(h) & 0x80000000u)),
+                                         __uint_as_float((304u - ex) << 23)));
+  long long m = ((long long)(hb & 0x7FFFFFu) << 29) + ((long long)n << 2);
+  // in the binade below or above h's: the mantissa in that binade's units
+  if ((unsigned int)(m >> 32) > 0xFFFFFu) m = m < 0 ? 2 * m : (m + (1ll << 52)) >> 1;
+  const unsigned long long sign = (unsigned long long)(__float_as_uint(h) & 0x80000000u) << 32;
+  return __longlong_as_double((long long)(sign | (unsigned long long)(((long long)(ex + 896u) << 52) + m)));
+}
+
+// A site's charge factor k and its FP32 head and tail.
+struct Factor {
+  double k;
+  float h, l;
+};
+
+// RN(k / RN(sqrt(r2))), the two correctly rounded FP64 operations, in 4 FP64
 // instructions.  The FP64 pipe executes 2 lanes a clock and SM, the FP32 and
 // integer pipes 128, so the reciprocal root y is refined to ~2^-45 in FP32 (the
 // residual 1 - r2 y0^2 of the hardware's estimate with the error of every
-// product) and put together with integer operations; one FP64 residual each
-// then gives the root and the quotient to ~2^-89 before their final rounding
-// (Markstein, IBM J. Res. Dev. 34, 1990).  Sets bad for r2 outside [2^-60, 2^62).
-__device__ __forceinline__ double quotient_root(double k, double r2, bool& bad) {
+// product), s0 = r2 y and q0 = k y are formed as FP32 pairs, and all three are put
+// together with integer operations; one FP64 residual each then gives the root
+// and the quotient to ~2^-86 before their final rounding (Markstein, IBM J.
+// Res. Dev. 34, 1990).  Sets bad for r2 outside [2^-60, 2^62).
+__device__ __forceinline__ double quotient_root(const Factor& f, double r2, bool& bad) {
   const unsigned int hi = (unsigned int)__double2hiint(r2), lo = (unsigned int)__double2loint(r2);
   bad = bad || (hi - 0x3C300000u) >= 0x07A00000u;
   // r2 = a + b: the leading 24 bits and the other 29, rounded
@@ -189,40 +210,41 @@ __device__ __forceinline__ double quotient_root(double k, double r2, bool& bad) 
   const float y0 = rsqrtf(a);
   const float p = __fmul_rn(y0, y0), pe = __fmaf_rn(y0, y0, -p);
   const float t = __fmaf_rn(-b, p, __fmaf_rn(-a, pe, __fmaf_rn(-a, p, 1.f)));
-  const float c = __fmul_rn(__fmul_rn(y0, t), __fmaf_rn(0.375f, t, 0.5f));
-  // y = y0 + c, c as a fixed-point number of units 2^-50 of y0's binade
-  const unsigned int yb = __float_as_uint(y0);
-  const int n = __float2int_rn(__fmul_rn(c, __uint_as_float((304u - (yb >> 23)) << 23)));
-  long long m = ((long long)(yb & 0x7FFFFFu) << 29) + ((long long)n << 2);
-  // y in the binade below or above y0's: its mantissa in that binade's units
-  if ((unsigned int)(m >> 32) > 0xFFFFFu) m = m < 0 ? 2 * m : (m + (1ll << 52)) >> 1;
-  const long long ybits = ((long long)((yb >> 23) + 896u) << 52) + m;
-  const double y = __longlong_as_double(ybits), half_y = __longlong_as_double(ybits - (1ll << 52));
-  const double s0 = __dmul_rn(r2, y);
+  const float c = __fmul_rn(__fmul_rn(y0, t), __fmaf_rn(0.375f, t, 0.5f));  // y = y0 + c
+  const float sh = __fmul_rn(a, y0);
+  const float sl = __fmaf_rn(b, y0, __fmaf_rn(a, c, __fmaf_rn(a, y0, -sh)));
+  const float qh = __fmul_rn(f.h, y0);
+  const float ql = __fmaf_rn(f.l, y0, __fmaf_rn(f.h, c, __fmaf_rn(f.h, y0, -qh)));
+  const double y = double_of(y0, c), s0 = double_of(sh, sl), q0 = f.h != 0.f ? double_of(qh, ql) : 0.0;
+  const double half_y = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));
   const double s = fma(fma(-s0, s0, r2), half_y, s0);
-  const double q0 = __dmul_rn(k, y);
-  return fma(fma(-q0, s, k), y, q0);
+  return fma(fma(-q0, s, f.k), y, q0);
 }
 
 // One thread per point, theta_a and kPhis values of phi_b, both phi halves.
 // Bound by the FP64 pipe: the two H positions of a node and of its mirror image
 // under phi -> 2 pi - phi share their coordinates, and all of a theta their z,
-// which leaves 4.3 operations for a squared distance, 6 for the term and 1 to
+// which leaves 4.3 operations for a squared distance, 4 for the term and 1 to
 // add it, against 29 with one thread per node and the compiler's square root
-// and division: 303 instead of 698 ms at 41^3, 30 x 60 nodes, 60 sites (267 ms
-// at the pipe's rate).  The results are the same bits.
+// and division: 247 instead of 698 ms at 41^3, 30 x 60 nodes, 60 sites (221 ms
+// at the pipe's rate; 303 ms with the starting root and quotient formed in FP64).  The results are the same bits.
 constexpr int kPhis = 3;
 __global__ void __launch_bounds__(kThreads) k_potential_alavi(AtomSet atoms, const double* xg, const double* yg,
                                                               const double* zg, int nx, int ny, long long npts,
                                                               int na, int nb, const double* hdir, const double* cm,
                                                               double ceiling, double* v1, double* v2) {
-  __shared__ double sxyz[3 * kMaxAtoms], sq[kMaxAtoms], skq[kMaxAtoms];
+  __shared__ double sxyz[3 * kMaxAtoms], sq[kMaxAtoms];
+  __shared__ Factor skq[kMaxAtoms];
   for (int i = threadIdx.x; i < atoms.n; i += blockDim.x) {
     sxyz[3 * i] = atoms.xyz[3 * i];
     sxyz[3 * i + 1] = atoms.xyz[3 * i + 1];
     sxyz[3 * i + 2] = atoms.xyz[3 * i + 2];
     sq[i] = atoms.q[i];
-    skq[i] = __dmul_rn(__dmul_rn(kCoulombK, atoms.q_h), atoms.q[i]);
+    const double k = __dmul_rn(__dmul_rn(kCoulombK, atoms.q_h), atoms.q[i]);
+    const float h = (float)k;
+    // a factor outside [2^-40, 2^40), but for 0, takes the plain operations (skq.h = NaN)
+    const bool plain = !(k == 0.0 || (fabs(k) >= 0x1p-40 && fabs(k) < 0x1p40));
+    skq[i] = Factor{k, plain ? __int_as_float(0x7fc00000) : h, (float)(k - (double)h)};
   }
   __syncthreads();
   const int nbg = (nb + kPhis - 1) / kPhis, nab = na * nb;
@@ -247,7 +269,9 @@ __global__ void __launch_bounds__(kThreads) k_potential_alavi(AtomSet atoms, con
   }
   bool bad = false;
   for (int w = 0; w < atoms.n; ++w) {
-    const double sx = sxyz[3 * w], sy = sxyz[3 * w + 1], sz = sxyz[3 * w + 2], kq = skq[w];
+    const double sx = sxyz[3 * w], sy = sxyz[3 * w + 1], sz = sxyz[3 * w + 2];
+    const Factor kq = skq[w];
+    bad = bad || !(kq.h == kq.h);
     auto square = [](double s, double q) {
       const double d = __dsub_rn(s, q);
       return __dmul_rn(d, d);
