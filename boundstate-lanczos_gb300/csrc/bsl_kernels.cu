@@ -329,17 +329,16 @@ __global__ void k_potential_iso(const double* xg, const double* yg, const double
 // potential blocks: one CTA per grid point.
 //   F[a][m,m'] = sum_b w_b (T1_m(b) T1_m'(b) V1(a,b) + T2_m(b) T2_m'(b) V2(a,b))
 //   B[s,s']   = sum_a w_a L_s(a) L_s'(a) F[a][m_s, m_s']
+// Bound by the FP64 pipe, so the products of the factors come from tables: 3
+// operations per phi node and pair instead of 5, 1 per theta node and element
+// instead of 3, the same bits (23.8 against 40.9 ms at 41^3, 30 x 60 nodes, 21
+// functions; 19.6 ms at the pipe's rate).
 // ---------------------------------------------------------------------------
 struct BlockTables {
-  const double* trig1;  // [nm][nb]
-  const double* trig2;
-  const double* leg;    // [nn][na]
-  const double* wa;     // [na]
-  const double* wb;     // [nb]
-  const int2* mpair;    // [nmtri] (mi, mj), mi <= mj
-  const int2* spair;    // [ntri] (s, s')
+  const double2* trig;  // [nb][nmtri]: T1_m T1_m' and T2_m T2_m' of pair (m, m'), m <= m', sqrt(w_b) in each T
+  const double* leg;    // [na][ntri]: w_a L_s L_s'
   const int* fidx;      // [ntri] index into the mpair list of (m_s, m_s') sorted
-  int na, nb, nm, nmtri, nn, ntri;
+  int na, nb, nmtri, ntri;
 };
 
 __global__ void k_vblocks(BlockTables bt, const double* v1, const double* v2, long long npts, double* vb64,
@@ -348,43 +347,33 @@ __global__ void k_vblocks(BlockTables bt, const double* v1, const double* v2, lo
   const int na = bt.na, nb = bt.nb, nab = na * nb;
   double* sV1 = smem;
   double* sV2 = sV1 + nab;
-  double* sT1 = sV2 + nab;
-  double* sT2 = sT1 + bt.nm * nb;
-  double* sL = sT2 + bt.nm * nb;
-  double* sF = sL + bt.nn * na;
+  double* sF = sV2 + nab;  // [na][nmtri]
   const long long p = blockIdx.x;
   for (int e = threadIdx.x; e < nab; e += blockDim.x) {
     sV1[e] = v1[p * nab + e];
     sV2[e] = v2[p * nab + e];
   }
-  for (int e = threadIdx.x; e < bt.nm * nb; e += blockDim.x) {
-    const int b = e % nb;
-    sT1[e] = bt.trig1[e] * sqrt(bt.wb[b]);
-    sT2[e] = bt.trig2[e] * sqrt(bt.wb[b]);
-  }
-  for (int e = threadIdx.x; e < bt.nn * na; e += blockDim.x) sL[e] = bt.leg[e];
   __syncthreads();
   for (int e = threadIdx.x; e < na * bt.nmtri; e += blockDim.x) {
     const int a = e / bt.nmtri;
-    const int2 mm = bt.mpair[e % bt.nmtri];
-    const double* t1a = sT1 + mm.x * nb;
-    const double* t1b = sT1 + mm.y * nb;
-    const double* t2a = sT2 + mm.x * nb;
-    const double* t2b = sT2 + mm.y * nb;
+    const double2* t = bt.trig + (e - a * bt.nmtri);
     const double* va = sV1 + a * nb;
     const double* vb = sV2 + a * nb;
     double f = 0.0;
-    for (int b = 0; b < nb; ++b) f += t1a[b] * t1b[b] * va[b] + t2a[b] * t2b[b] * vb[b];
+#pragma unroll 4
+    for (int b = 0; b < nb; ++b) {
+      const double2 w = __ldg(t + (size_t)b * bt.nmtri);
+      f += w.x * va[b] + w.y * vb[b];
+    }
     sF[e] = f;
   }
   __syncthreads();
   for (int t = threadIdx.x; t < bt.ntri; t += blockDim.x) {
-    const int2 ss = bt.spair[t];
-    const int fi = bt.fidx[t];
-    const double* la = sL + ss.x * na;
-    const double* lb = sL + ss.y * na;
+    const double* l = bt.leg + t;
+    const double* f = sF + bt.fidx[t];
     double acc = 0.0;
-    for (int a = 0; a < na; ++a) acc += bt.wa[a] * la[a] * lb[a] * sF[a * bt.nmtri + fi];
+#pragma unroll 4
+    for (int a = 0; a < na; ++a) acc += __ldg(l + (size_t)a * bt.ntri) * f[a * bt.nmtri];
     vb64[(long long)t * npts + p] = acc;
     vb32[((p / tile_pts) * bt.ntri + t) * tile_pts + p % tile_pts] = (float)acc;
   }
@@ -1018,42 +1007,41 @@ int dev_vblocks(bsl_handle* h) {
       if (ma > mb) std::swap(ma, mb);
       fidx.push_back(mindex[(size_t)ma * nm + mb]);
     }
-  double *dt1, *dt2, *dleg, *dwa, *dwb;
-  int2 *dmp, *dsp;
-  int* dfi;
-  BSL_CUDA(cudaMalloc(&dt1, t.trig1.size() * 8));
-  BSL_CUDA(cudaMalloc(&dt2, t.trig2.size() * 8));
-  BSL_CUDA(cudaMalloc(&dleg, t.leg.size() * 8));
-  BSL_CUDA(cudaMalloc(&dwa, t.gl_w.size() * 8));
-  BSL_CUDA(cudaMalloc(&dwb, t.gc_w.size() * 8));
-  BSL_CUDA(cudaMalloc(&dmp, mpair.size() * sizeof(int2)));
-  BSL_CUDA(cudaMalloc(&dsp, spair.size() * sizeof(int2)));
-  BSL_CUDA(cudaMalloc(&dfi, fidx.size() * sizeof(int)));
-  BSL_CUDA(cudaMemcpy(dt1, t.trig1.data(), t.trig1.size() * 8, cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dt2, t.trig2.data(), t.trig2.size() * 8, cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dleg, t.leg.data(), t.leg.size() * 8, cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dwa, t.gl_w.data(), t.gl_w.size() * 8, cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dwb, t.gc_w.data(), t.gc_w.size() * 8, cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dmp, mpair.data(), mpair.size() * sizeof(int2), cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dsp, spair.data(), spair.size() * sizeof(int2), cudaMemcpyHostToDevice));
-  BSL_CUDA(cudaMemcpy(dfi, fidx.data(), fidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-  BlockTables bt{dt1, dt2, dleg, dwa, dwb, dmp, dsp, dfi, t.na, t.nb, nm, nmtri, t.nn, ntri};
-  const size_t smem = 8 * ((size_t)2 * t.na * t.nb + (size_t)2 * nm * t.nb + (size_t)t.nn * t.na +
-                           (size_t)t.na * nmtri);
-  int rc = BSL_OK;
-  if (smem > 220 * 1024) {
-    rc = fail(BSL_ERR_UNSUPPORTED, "angular quadrature too large for the block assembly kernel");
-  } else {
-    cudaFuncSetAttribute(k_vblocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_vblocks<<<(unsigned)t.npts, kThreads, smem, d.stream>>>(bt, d.v1, d.v2, t.npts, d.vb64, d.vb32,
-                                                               vstream_tile_points());
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(d.stream);
-    if (e != cudaSuccess) rc = cuda_fail(e, "potential block assembly");
+  // the products of the factors, formed once for all points
+  std::vector<double2> trig((size_t)t.nb * nmtri);
+  std::vector<double> leg((size_t)t.na * ntri);
+  for (int b = 0; b < t.nb; ++b) {
+    const double w = std::sqrt(t.gc_w[b]);
+    for (int k = 0; k < nmtri; ++k) {
+      const size_t x = (size_t)mpair[k].x * t.nb + b, y = (size_t)mpair[k].y * t.nb + b;
+      const double x1 = t.trig1[x] * w, y1 = t.trig1[y] * w, x2 = t.trig2[x] * w, y2 = t.trig2[y] * w;
+      trig[(size_t)b * nmtri + k] = make_double2(x1 * y1, x2 * y2);
+    }
   }
-  cudaFree(dt1); cudaFree(dt2); cudaFree(dleg); cudaFree(dwa); cudaFree(dwb);
-  cudaFree(dmp); cudaFree(dsp); cudaFree(dfi);
-  return rc;
+  for (int a = 0; a < t.na; ++a)
+    for (int k = 0; k < ntri; ++k)
+      leg[(size_t)a * ntri + k] =
+          t.gl_w[a] * t.leg[(size_t)spair[k].x * t.na + a] * t.leg[(size_t)spair[k].y * t.na + a];
+  // the largest quadrature the assembly takes (the grid values, tables and one
+  // sum per theta and pair of m within 220 KiB)
+  if (8 * ((size_t)2 * t.na * t.nb + (size_t)2 * nm * t.nb + (size_t)t.nn * t.na + (size_t)t.na * nmtri) > 220 * 1024)
+    return fail(BSL_ERR_UNSUPPORTED, "angular quadrature too large for the block assembly kernel");
+  Uploads up;
+  double2* dtrig;
+  double* dleg;
+  int* dfi;
+  cudaError_t e;
+  if ((e = up.put(&dtrig, trig)) != cudaSuccess || (e = up.put(&dleg, leg)) != cudaSuccess ||
+      (e = up.put(&dfi, fidx)) != cudaSuccess)
+    return cuda_fail(e, "potential block tables");
+  const BlockTables bt{dtrig, dleg, dfi, t.na, t.nb, nmtri, ntri};
+  const size_t smem = 8 * ((size_t)2 * t.na * t.nb + (size_t)t.na * nmtri);
+  cudaFuncSetAttribute(k_vblocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_vblocks<<<(unsigned)t.npts, kThreads, smem, d.stream>>>(bt, d.v1, d.v2, t.npts, d.vb64, d.vb32,
+                                                             vstream_tile_points());
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(d.stream);
+  return e == cudaSuccess ? BSL_OK : cuda_fail(e, "potential block assembly");
 }
 
 int dev_hv(bsl_handle* h, const double* v, double* u, cudaStream_t s) {
