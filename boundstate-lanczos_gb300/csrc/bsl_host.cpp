@@ -776,9 +776,11 @@ int bsl_hv_apply(bsl_handle* h, const double* vec, double* uec) {
   BSL_CUDA(cudaStreamSynchronize(s));
   int st[4] = {0, 0, 0, 0};
   BSL_CUDA(cudaMemcpy(st, d.status, sizeof(st), cudaMemcpyDeviceToHost));
-  if (st[2] || st[3])
+  if (st[2] || st[3]) {
+    cudaMemset(d.status, 0, sizeof(st));  // reported: later calls start clean
     return fail(BSL_ERR_CUDA, st[2] ? "potential-block stream: a bulk copy did not complete within its time limit"
                                     : "tensor-core kinetic: an MMA did not complete within its time limit");
+  }
   return BSL_OK;
 }
 

@@ -145,6 +145,8 @@ int init_state(bsl_handle* h, int start, unsigned long long seed) {
 int check_status(bsl_handle* h) {
   int st[4] = {0, 0, 0, 0};
   BSL_CUDA(cudaMemcpy(st, h->d.status, 4 * sizeof(int), cudaMemcpyDeviceToHost));
+  // a time-out is reported once: kernels launched outside a run (H v) read the words too
+  if (st[2] || st[3]) BSL_CUDA(cudaMemset(h->d.status, 0, 4 * sizeof(int)));
   if (st[2]) return fail(BSL_ERR_CUDA, "potential-block stream: a bulk copy did not complete within its time limit");
   if (st[3]) return fail(BSL_ERR_CUDA, "tensor-core kinetic: an MMA did not complete within its time limit");
   if (st[0]) return fail(BSL_ERR_BREAKDOWN, "Lanczos breakdown at iteration " + std::to_string(st[1]) +
@@ -545,6 +547,8 @@ int run_batch(bsl_handle** hs, int n, int niter, int start, unsigned long long s
     }
     for (int b = 0; b < n; ++b) hs[b]->last_ms_per_iter = batch_ms / niter;
   }
+  std::string first_error;
+  rc = BSL_OK;
   for (int b = 0; b < n; ++b) {
     bsl_handle* h = hs[b];
     cudaSetDevice(h->p.device);
@@ -559,9 +563,13 @@ int run_batch(bsl_handle** hs, int n, int niter, int start, unsigned long long s
       beta[b][j] = hist[d.hist_cap + j];
       beta2[b][j] = hist[2 * (size_t)d.hist_cap + j];
     }
-    if ((rc = check_status(h))) return rc;
+    const int st = check_status(h);  // of every problem: each word is cleared once reported
+    if (st && !rc) {
+      rc = st;
+      first_error = bsl_last_error();
+    }
   }
-  return BSL_OK;
+  return rc ? fail(rc, first_error) : BSL_OK;
 }
 
 }  // namespace

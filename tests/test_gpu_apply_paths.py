@@ -86,6 +86,24 @@ def test_fp64_hv_of_non_finite_and_zero_vectors(bsl, tmp_path):
         h.close()
 
 
+def test_fp64_hv_after_a_reported_time_out(bsl, tmp_path):
+    """The FP64 tensor-core kinetic leaves when a time-out is recorded; once a run
+    has reported it, H v works again."""
+    h = bsl.Hamiltonian(write_case(str(tmp_path), (26, 26, 26), 5, "Odd"), CALC, precision="fp64")
+    try:
+        v = np.random.default_rng(2).standard_normal(h.basis_size)
+        ref, u = np.zeros_like(v), np.zeros_like(v)
+        h.hv(v, ref)
+        h.inject_timeout(2)
+        with pytest.raises(bsl.BslError):
+            h.lanczos(3)
+        h.inject_timeout(0)
+        h.hv(v, u)
+        assert np.array_equal(u, ref)
+    finally:
+        h.close()
+
+
 # one launch up to 16 points: smallest grids, planes of a full and of a broken warp
 # count, unequal z, the last size of the range and the first beyond it
 @pytest.mark.parametrize("n,nz,l_max,sym", [(4, 4, 4, "Even"), (5, 16, 5, "Odd"), (11, 6, 3, "Odd"), (7, 9, 3, "All"),
