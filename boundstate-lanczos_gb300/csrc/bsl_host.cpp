@@ -762,20 +762,26 @@ int bsl_hv_apply(bsl_handle* h, const double* vec, double* uec) {
   DeviceState& d = h->d;
   const size_t Df = (size_t)bsl_basis_size(h);
   int rc;
-  if (!d.ref_vec && ((rc = dalloc(&d.ref_vec, Df, "staging")) || (rc = dalloc(&d.ref_out, Df, "staging")))) return rc;
+  if ((rc = ensure_staging(h))) return rc;
   cudaStream_t s = d.stream;
   // the device Lanczos vectors serve as packed scratch here
   h->state_pairs = -1;
   BSL_CUDA(cudaMemcpyAsync(d.ref_vec, vec, Df * sizeof(double), cudaMemcpyHostToDevice, s));
-  BSL_CUDA(cudaMemcpyAsync(d.ref_out, uec, Df * sizeof(double), cudaMemcpyHostToDevice, s));
+  BSL_CUDA(cudaEventRecord(d.vec_in, s));
   if ((rc = dev_gather_packed(h, d.ref_vec, d.vec, s))) return rc;
   if ((rc = dev_hv(h, d.vec, d.rvec, s))) return rc;
+  // uec comes in on a second stream while H v runs (issued after it: a copy from
+  // pageable memory may hold the host until it is done)
+  BSL_CUDA(cudaStreamWaitEvent(d.copy_stream, d.vec_in, 0));
+  BSL_CUDA(cudaMemcpyAsync(d.ref_out, uec, Df * sizeof(double), cudaMemcpyHostToDevice, d.copy_stream));
+  BSL_CUDA(cudaEventRecord(d.copy_done, d.copy_stream));
+  BSL_CUDA(cudaStreamWaitEvent(s, d.copy_done, 0));
   // uec += H vec on the symmetry block; the reference adds S_n (...) = 0 elsewhere
   if ((rc = dev_scatter_full(h, d.rvec, d.ref_out, s))) return rc;
   BSL_CUDA(cudaMemcpyAsync(uec, d.ref_out, Df * sizeof(double), cudaMemcpyDeviceToHost, s));
-  BSL_CUDA(cudaStreamSynchronize(s));
   int st[4] = {0, 0, 0, 0};
-  BSL_CUDA(cudaMemcpy(st, d.status, sizeof(st), cudaMemcpyDeviceToHost));
+  BSL_CUDA(cudaMemcpyAsync(st, d.status, sizeof(st), cudaMemcpyDeviceToHost, s));
+  BSL_CUDA(cudaStreamSynchronize(s));
   if (st[2] || st[3]) {
     cudaMemset(d.status, 0, sizeof(st));  // reported: later calls start clean
     return fail(BSL_ERR_CUDA, st[2] ? "potential-block stream: a bulk copy did not complete within its time limit"

@@ -334,6 +334,8 @@ int dev_vblocks_bf16(bsl_handle* h);
 int gaunt_coefficient_count(const bsl_handle* h);
 int dev_gaunt_coeffs(bsl_handle* h, double* residual, double* vmax);
 
+// host-layout staging buffers, the second copy stream and its events (bsl_lanczos.cpp)
+int ensure_staging(bsl_handle* h);
 // the cached iteration graph (bsl_lanczos.cpp)
 void release_iteration_graph(DeviceState& d);
 

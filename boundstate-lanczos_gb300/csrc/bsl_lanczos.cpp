@@ -30,6 +30,20 @@ int dev_fill(double* x, long long L, double val, cudaStream_t s);
 int dev_to_f32(const double* x, float* y, long long n, cudaStream_t s);
 int dev_to_pair(double* x, long long n, cudaStream_t s);
 
+int ensure_staging(bsl_handle* h) {
+  DeviceState& d = h->d;
+  if (!d.copy_stream) {
+    BSL_CUDA(cudaStreamCreateWithFlags(&d.copy_stream, cudaStreamNonBlocking));
+    BSL_CUDA(cudaEventCreateWithFlags(&d.copy_done, cudaEventDisableTiming));
+    BSL_CUDA(cudaEventCreateWithFlags(&d.vec_in, cudaEventDisableTiming));
+  }
+  if (d.ref_vec) return BSL_OK;
+  const size_t Df = (size_t)bsl_basis_size(h);
+  BSL_CUDA(cudaMalloc(&d.ref_vec, Df * sizeof(double) + 16));
+  BSL_CUDA(cudaMalloc(&d.ref_out, Df * sizeof(double) + 16));
+  return BSL_OK;
+}
+
 namespace {
 
 // The history buffer grows in steps of kHistStep iterations, so runs of
@@ -67,20 +81,6 @@ double* mapped_host(double* p) {
     return nullptr;
   }
   return a.type == cudaMemoryTypeHost ? static_cast<double*>(a.devicePointer) : nullptr;
-}
-
-int ensure_staging(bsl_handle* h) {
-  DeviceState& d = h->d;
-  if (!d.copy_stream) {
-    BSL_CUDA(cudaStreamCreateWithFlags(&d.copy_stream, cudaStreamNonBlocking));
-    BSL_CUDA(cudaEventCreateWithFlags(&d.copy_done, cudaEventDisableTiming));
-    BSL_CUDA(cudaEventCreateWithFlags(&d.vec_in, cudaEventDisableTiming));
-  }
-  if (d.ref_vec) return BSL_OK;
-  const size_t Df = (size_t)bsl_basis_size(h);
-  BSL_CUDA(cudaMalloc(&d.ref_vec, Df * sizeof(double) + 16));
-  BSL_CUDA(cudaMalloc(&d.ref_out, Df * sizeof(double) + 16));
-  return BSL_OK;
 }
 
 uint64_t splitmix64(uint64_t* s) {
