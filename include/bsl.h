@@ -397,7 +397,8 @@ int bsl_selftest_tensor_core(double* max_abs_err);
    kernel on the library's stream and writes the average milliseconds per
    launch of the stages {kinetic x/y, kinetic z, potential apply + alpha,
    update + beta, normalise + swap} into ms[0..4]; names[i] (optional) receives
-   the kernel name of stage i (static strings). */
+   the kernel name of stage i (static strings).  Where one launch forms the whole
+   kinetic, the second stage holds no launch. */
 int bsl_stage_times(bsl_handle* h, int iters, double* ms, const char** names);
 
 /* Launch-shape autotuner, with no counterpart in the reference: times
