@@ -328,8 +328,8 @@ void free_device(DeviceState& d) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (d.vpair) cudaFree(d.vpair);
-  if (d.kxy_slices) cudaFree(d.kxy_slices);
-  if (d.kz_slices) cudaFree(d.kz_slices);
+  if (d.kin_slices) cudaFree(d.kin_slices);
+  if (d.ukin_z) cudaFree(d.ukin_z);
   if (d.tx_slices32) cudaFree(d.tx_slices32);
   if (d.tz_slices32) cudaFree(d.tz_slices32);
   if (d.kxy_slices64) cudaFree(d.kxy_slices64);
@@ -434,10 +434,10 @@ int hv_prep(const bsl_hv_params* params, const Cage* cage, bsl_handle** out) {
   if ((rc = upload(&d.kz_head, hi, "Tz")) || (rc = upload(&d.kz_band, lo, "Tz"))) return bail(rc);
   if (kinetic_tc_supported(t)) {
     std::vector<uint16_t> sl;
-    kinetic_smem_image(t.tx, t.nx, true, &sl, &d.e_txy);
-    if ((rc = upload(&d.kxy_slices, sl, "Tx"))) return bail(rc);
-    kinetic_smem_image(t.tz, t.nz, false, &sl, &d.e_tz);
-    if ((rc = upload(&d.kz_slices, sl, "Tz"))) return bail(rc);
+    kinetic_tc_image(t, &sl, &d.kin_tz_tile, &d.e_txy, &d.e_tz);
+    d.kin_image16 = (int)(sl.size() * sizeof(uint16_t) / 16);
+    if ((rc = upload(&d.kin_slices, sl, "T"))) return bail(rc);
+    if (kin_tc_one_launch(h) && (rc = dalloc(&d.ukin_z, (size_t)t.npts * t.nn, "kinetic work"))) return bail(rc);
     std::vector<float> sf;
     kinetic_slices_f32(t.tx, t.nx, &sf);
     if ((rc = upload(&d.tx_slices32, sf, "Tx"))) return bail(rc);
@@ -711,7 +711,7 @@ int bsl_set_precision(bsl_handle* h, int precision) {
 int bsl_set_kinetic_engine(bsl_handle* h, int engine) {
   if (!h) return fail(BSL_ERR_STATE, "null handle");
   if (engine != BSL_KIN_SIMT && engine != BSL_KIN_TENSOR) return fail(BSL_ERR_INPUT, "unknown kinetic engine");
-  if (engine == BSL_KIN_TENSOR && !h->d.kxy_slices)
+  if (engine == BSL_KIN_TENSOR && !h->d.kin_slices)
     return fail(BSL_ERR_UNSUPPORTED, "tensor-core kinetic needs at most 64 points per axis and equal x and y axes");
   if (engine != h->kinetic_engine) h->state_pairs = -1;  // the FP32 copy of v is kept for the CUDA-core engine only
   h->kinetic_engine = engine;

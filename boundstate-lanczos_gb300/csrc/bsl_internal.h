@@ -97,8 +97,9 @@ struct DeviceState {
   float *kx_band = nullptr, *ky_band = nullptr, *kz_band = nullptr;
   // fixed-point FP16 slices of T (5 zero-padded 64 x 64 tiles) and their scale
   // exponents, for the tensor-core kinetic
-  uint16_t *kxy_slices = nullptr, *kz_slices = nullptr;
-  int e_txy = 0, e_tz = 0;
+  uint16_t* kin_slices = nullptr;  // of x/y, then of z unless the same (kinetic_tc_image)
+  int kin_image16 = 0, kin_tz_tile = 0, e_txy = 0, e_tz = 0;
+  float2* ukin_z = nullptr;        // one-launch tensor-core kinetic: the z part (x/y in ukin)
   float *tx_slices32 = nullptr, *tz_slices32 = nullptr;  // the slices as FP32 integers (bsl_small.cu)
   // the same for the FP64 path: seven slices (bsl_kinetic_tc64.cu)
   uint16_t *kxy_slices64 = nullptr, *kz_slices64 = nullptr;
@@ -244,6 +245,9 @@ void kinetic_smem_image64(const std::vector<double>& T, int n, bool with_zero_ti
                           int* e_t);
 int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s);
 bool kin_f64_tensor(const bsl_handle* h);
+void kinetic_tc_image(const Tables& t, std::vector<uint16_t>* image, int* tz_tile, int* e_txy, int* e_tz);
+// whether launch_kin_xy_tc forms all three contractions (z in d.ukin_z) and launch_kin_z_tc nothing
+bool kin_tc_one_launch(const bsl_handle* h);
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 int launch_kin_z_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 // grouped tensor-core kinetic over several problems: per-problem argument
@@ -264,6 +268,7 @@ struct StreamArgs {
   const float2* vpair;  // mode 0 of the tensor-core kinetic: v as pairs, whose heads take its place
   const double* vec;    // FP64 v (alpha dot product, extra coordinate)
   const float2* ukin;   // kinetic (hi, lo) pairs
+  const float2* ukin_z; // its z part where it is kept apart (one-launch tensor-core kinetic), or null
   const float* rot_hi;  // rotor energies, head and tail
   const float* rot_lo;
   double* out;          // mode 0: u = H v; mode 1: the Lanczos r buffer (r += c H v)

@@ -790,6 +790,8 @@ StreamArgs vstream_args(bsl_handle* h, const double* v, double* out) {
   a.v32 = d.v32;
   a.vec = v;
   a.ukin = reinterpret_cast<const float2*>(d.ukin);
+  const bool apart = h->kinetic_engine == BSL_KIN_TENSOR && !kin_small_supported(h) && kin_tc_one_launch(h);
+  a.ukin_z = apart ? d.ukin_z : nullptr;
   a.rot_hi = d.rot_hi;
   a.rot_lo = d.rot_lo;
   a.out = out;
@@ -1205,8 +1207,10 @@ const char* dev_stage_name(bsl_handle* h, int i) {
   static const char* nmx[4] = {"k_kin_xy_split", "k_kin_z_split", "k_vstream<NN>", "k_update_pair"};
   static const char* nts[2] = {"k_kin_small", "(in k_kin_small)"};
   static const char* ntc[4] = {"k_kin_xy_tc", "k_kin_z_tc", "k_vstream<NN>", "k_update_stream"};
+  static const char* nto[2] = {"k_kin_xyz_tc", "(in k_kin_xyz_tc)"};
   if (!mixed) return i < 2 && kin_f64_tensor(h) ? n64t[i] : n64[i];
   if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)) return nts[i];
+  if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_tc_one_launch(h)) return nto[i];
   if (fused_iterations(h) && i >= 2)
     return i == 2 ? "k_vapply_light<NN>" : h->vformat == BSL_VFMT_GAUNT ? "k_vstream<NN,coefficients,update>"
                                                                         : "k_vstream<NN,fp32,update>";

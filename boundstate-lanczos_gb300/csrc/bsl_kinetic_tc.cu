@@ -8,15 +8,17 @@
 // Work unit: a pair of planes.  The accumulator D has M = 128 rows (p, x) --
 // plane p of the pair, grid column x -- and N = 64 columns (the other in-plane
 // index), K = 64 per contraction:
-//   x and y (k_kin_xy_tc), planes (y, x) of fixed (s, z); both directions
+//   x and y, planes (y, x) of fixed (s, z); both directions
 //     accumulate into the same D[(p, x)][y]:
 //       y:  sum_q v_p(q, x) Ty[y][q]      A = v tile read MN-major, B = T
 //       x:  sum_q Tx[x][q] v_p(y, q)      A = diag(Tx, Tx) over K = (p', q), B = v tile
 //     (the block-diagonal A is two 128-row tiles [T; 0] and [0; T] made from the
 //     T tile and zero tiles laid out around it);
-//   z (k_kin_z_tc), planes (z, x) of fixed (s, y):
+//   z, planes (z, x) of fixed (s, y):
 //       sum_q v_p(q, x) Tz[z][q]           A = v tile read MN-major, B = T
-//     and the result is added to the x/y result.
+// k_kin_tc<kXY> forms the first and k_kin_tc<kZ> adds the second to it; small
+// problems take k_kin_tc<kAll>, which forms both in one launch and leaves the z
+// part in a buffer of its own for the apply to add (kin_tc_one_launch).
 // Every v tile is stored once, row by row as it lies in memory (64 FP16 per
 // 128-byte swizzled row), and read by both terms; the output rows of D are
 // grid columns, so the epilogue's stores are coalesced along x.
@@ -71,16 +73,17 @@ constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kMaxItems = 64 * 16 / kProdThreads;  // (row, 4-column group) items per producer thread
 
 struct KinTC {
-  const uint4* timage;      // the T tiles as laid out in shared memory (kinetic_smem_image)
+  const uint4* timage;      // the T tiles as laid out in shared memory: Z T0 .. T3 Z (x/y), then Tz unless it is the same
   int timage16;             // its size in 16-byte units
-  int e_t;                  // T = 2^(e_t - 8) (b1 + 2^-9 b2 + 2^-18 b3 + 2^-27 b4)
+  int tz_tile;              // first tile of Tz's slices
+  int e_txy, e_tz;          // T = 2^(e_t - 8) (b1 + 2^-9 b2 + 2^-18 b3 + 2^-27 b4)
   const float2* v;          // the Lanczos v as double-float pairs
-  float2* out;
-  int nx, ny, nz, nplanes;
+  float2 *out_xy, *out_z;   // Tx v + Ty v; Tz v
+  int nx, ny, nz, nn;
   int* status;
   int nslices;              // slices of v and of T kept (1-4; 4 = exact), classes k + l < nslices
-  // x/y of a graph-replayed iteration: the first CTA's epilogue warps finish
-  // the previous update's deferred beta (null: nothing deferred)
+  // graph-replayed iterations: the first CTA's epilogue warps finish the previous
+  // update's deferred beta (null: nothing deferred)
   double* fin_partials;
   double* scalars;
   double* hist;
@@ -126,31 +129,60 @@ __device__ __forceinline__ void load_pairs8(uint32_t taddr, float scale, int nsl
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-
 // Plane geometry: x/y planes are the contiguous (y, x) planes of fixed (s, z);
 // z planes are the (z, x) planes of fixed (s, y), rows nx * ny apart.
-template <bool kXY>
 struct Planes {
-  int nx, ny, nz, nplanes;
-  __device__ __forceinline__ long long base(int plane) const {
-    if (kXY) return (long long)plane * nx * ny;
+  int nx, ny, nz, nxy, nzx;  // nxy, nzx: planes of x/y and z
+  __device__ __forceinline__ int count(int z) const { return z ? nzx : nxy; }
+  __device__ __forceinline__ long long base(int z, int plane) const {
+    if (!z) return (long long)plane * nx * ny;
     return (long long)(plane / ny) * nz * nx * ny + (long long)(plane % ny) * nx;
   }
-  __device__ __forceinline__ long long row_stride() const { return kXY ? (long long)nx : (long long)nx * ny; }
-  __device__ __forceinline__ int rows() const { return kXY ? ny : nz; }
+  __device__ __forceinline__ int row_stride(int z) const { return z ? nx * ny : nx; }
+  __device__ __forceinline__ int rows(int z) const { return z ? nz : ny; }
 };
 
-// The CTA's plane pairs: p_first, p_first + p_stride, ... below p_end (the
-// single-problem launch strides over the grid; a grouped launch gives each CTA
-// one contiguous range of one problem).
-template <bool kXY>
+// The CTA's work items: the x/y and the z plane pair p of every p = first, first
+// + stride, ... below end, in turn (x/y pairs keep the tensor core busy, z pairs
+// the producers).
+template <int kKinds>
+struct Items {
+  int pair, z;  // z: 0 an x/y pair, 1 a z pair
+  int stride, end;
+  const Planes& pg;
+  __device__ __forceinline__ Items(const Planes& g, int first, int st, int e)
+      : pair(first),
+        z(kKinds == 2),
+        stride(st),
+        end(min(e, ((kKinds == 3 ? max(g.nxy, g.nzx) : g.count(kKinds == 2)) + 1) / 2)),
+        pg(g) {
+    skip();
+  }
+  __device__ __forceinline__ bool more() const { return pair < end; }
+  __device__ __forceinline__ void skip() {  // to the next pair that exists
+    while (pair < end && 2 * pair >= pg.count(z)) step();
+  }
+  __device__ __forceinline__ void step() {
+    if (kKinds != 3 || z) pair += stride;
+    if (kKinds == 3) z ^= 1;
+  }
+  __device__ __forceinline__ void next() {
+    step();
+    skip();
+  }
+};
+
+// What a launch forms: the x/y contractions, the z contraction added to them, or
+// all three with the z part in a buffer of its own (the apply adds it).
+enum Kinds { kXY = 1, kZ = 2, kAll = 3 };
+// T tiles in shared memory: Z T0 T1 T2 T3 Z of x/y, the slices of Tz, or both
+__host__ __device__ constexpr int t_tiles(int kinds) { return kinds == kXY ? kTS + 2 : kinds == kZ ? kTS : 2 * kTS + 2; }
+
+template <int kKinds>
 __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_stride, int p_end) {
   extern __shared__ uint8_t smraw[];
   uint8_t* sm = align1024(smraw);
-  // T tiles: x/y as Z T0 T1 T2 T3 Z (Z = zero tile), z as T0 T1 T2 T3; then
-  // the v stages
-  constexpr int kTTiles = kXY ? kTS + 2 : kTS;
-  uint8_t* V = sm + kTTiles * kTile;
+  uint8_t* V = sm + t_tiles(kKinds) * kTile;
   __shared__ uint64_t v_full[kStages], v_empty[kStages], acc_full[kStages], acc_empty[kStages], e_full[kStages];
   __shared__ uint64_t stages_zeroed, t_ready;  // setup by the epilogue warps
   __shared__ uint32_t tmem_slot;
@@ -158,8 +190,7 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
   __shared__ float red[2][kProdWarps];
   __shared__ int prod_go, failed, skip;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Planes<kXY> pg{a.nx, a.ny, a.nz, a.nplanes};
-  const int npairs = min((a.nplanes + 1) / 2, p_end);
+  const Planes pg{a.nx, a.ny, a.nz, a.nz * a.nn, a.ny * a.nn};
 
   // a kinetic time-out recorded before this launch (an earlier launch of the
   // run, or the host's injection) makes the CTA leave before it allocates
@@ -195,9 +226,6 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
     const int quad = warp & 3, half = warp >> 2;
     const int p = quad >> 1, x = ((quad & 1) << 5) + lane;
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-    const int ncols = pg.rows();
-    const long long cstride = pg.row_stride();
-    const int c_begin = half * 32, c_end = min(half * 32 + 32, ncols);
     {  // setup while the producers' first planes are in flight: zeroed v stages
        // (the producers write only the rows and 4-column groups that hold data,
        // so the padding of every stage stays zero), then the T tiles (a
@@ -223,26 +251,27 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
       tc::fence_smem_to_async();
       tc::mbar_arrive(&t_ready);
     }
-    pdl_wait();  // the output (and, for z, the values added to) belong to earlier kernels
-    if (kXY && a.fin_partials && p_first == 0) {
+    pdl_wait();  // the output (and, for z alone, the values added to) belong to earlier kernels
+    if (kKinds != kZ && a.fin_partials && p_first == 0) {
       __shared__ double fin8[kEpiWarps];
       finish_deferred_beta(a.fin_partials + kBetaPartials, a.fin_count, a.scalars, a.hist, a.hist_stride, a.jdev,
                            a.status, tid, kEpiThreads, 2, fin8);
     }
-    // z: the values the epilogue adds to, 8 columns of this thread's x
-    auto load8 = [&](long long ob, bool valid, int c0, float2 (&u0)[8]) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        u0[u] = (valid && c0 + u < c_end) ? a.out[ob + (c0 + u) * cstride] : make_float2(0.f, 0.f);
-    };
-    for (int it = 0, pair = p_first; pair < npairs; pair += p_stride, ++it) {
+    int it = 0;
+    for (Items<kKinds> w(pg, p_first, p_stride, p_end); w.more(); w.next(), ++it) {
       const int st = it & 1;
       const uint32_t par = (uint32_t)(it >> 1) & 1u;
-      const int plane = 2 * pair + p;
-      const bool valid = plane < a.nplanes && x < a.nx;
-      const long long ob = valid ? pg.base(plane) + x : 0;
-      float2 nxt[8];  // z: first chunk loaded while the products run
-      if (!kXY) load8(ob, valid, c_begin, nxt);
+      const int plane = 2 * w.pair + p;
+      const bool valid = plane < pg.count(w.z) && x < a.nx;
+      float2* out = (w.z ? a.out_z : a.out_xy) + (valid ? pg.base(w.z, plane) + x : 0);
+      const long long cstride = pg.row_stride(w.z);
+      const int c_begin = half * 32, c_end = min(half * 32 + 32, pg.rows(w.z));
+      float2 nxt[8];  // z alone: the values added to, the first chunk loaded while the products run
+      auto load8 = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) nxt[u] = (valid && c0 + u < c_end) ? out[(c0 + u) * cstride] : make_float2(0.f, 0.f);
+      };
+      if (kKinds == kZ) load8(c_begin);
       // lane 0 waits (bounded) and the warp leaves together on a timeout; once the
       // phases are complete every lane's own wait returns at once and orders its
       // reads after the producers' and the MMA thread's writes
@@ -256,70 +285,64 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
       tc::mbar_wait(&acc_full[st], par);
       tc::mbar_wait(&e_full[st], par);
       tc::fence_after_sync();
-      const float scale = pow2f(e_acc[st][p] + a.e_t - 16);
+      const float scale = pow2f(e_acc[st][p] + (w.z ? a.e_tz : a.e_txy) - 16);
       const uint32_t tbase = tmem + (uint32_t)st * kAccCols + lane_base;
 #pragma unroll 1
       for (int c0 = c_begin; c0 < c_end; c0 += 8) {
-        float2 v[8];
-        if (kXY) {
-          load_pairs8(tbase + (uint32_t)c0, scale, a.nslices, v);
-          if (valid)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (c0 + u < c_end) a.out[ob + (c0 + u) * cstride] = v[u];
-        } else {
-          float2 cur[8];
+        float2 v[8], cur[8];
+        if (kKinds == kZ) {
 #pragma unroll
           for (int u = 0; u < 8; ++u) cur[u] = nxt[u];
-          if (c0 + 8 < c_end) load8(ob, valid, c0 + 8, nxt);  // the next chunk, in flight meanwhile
-          load_pairs8(tbase + (uint32_t)c0, scale, a.nslices, v);
-          if (valid)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (c0 + u < c_end) a.out[ob + (c0 + u) * cstride] = df_add_fast(cur[u], v[u]);
+          if (c0 + 8 < c_end) load8(c0 + 8);  // the next chunk, in flight meanwhile
         }
+        load_pairs8(tbase + (uint32_t)c0, scale, a.nslices, v);
+        if (valid)
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (c0 + u < c_end) out[(c0 + u) * cstride] = kKinds == kZ ? df_add_fast(cur[u], v[u]) : v[u];
       }
       tc::fence_before_sync();
       tc::mbar_arrive(&acc_empty[st]);
     }
   } else if (warp < kMmaWarp) {
-    // ---- producers: item i = (row i / ncg, 4-column group i % ncg) of a plane,
-    // items ptid, ptid + 256, ...; the next plane's items are loaded into
-    // registers while this one is sliced ----
+    // ---- producers: piece i = (row i / ncg, 4-column group i % ncg) of a plane,
+    // pieces ptid, ptid + 256, ...; the next plane's pieces are loaded into
+    // registers while this one is sliced.  With both kinds the rows run to the longer
+    // of y and z: those beyond a plane's own are written as zeros ----
     const int ptid = tid - kEpiThreads, pw = ptid >> 5;
-    const int nrows = pg.rows(), nx = a.nx, ncg = (nx + 3) >> 2, nitems = nrows * ncg;
-    const long long rstride = pg.row_stride();
-    // per item: offset in a plane, offset in a shared-memory tile, values present
-    int goff[kMaxItems], cnt[kMaxItems];
+    const int nx = a.nx, ncg = (nx + 3) >> 2, nrows = kKinds == kAll ? max(a.ny, a.nz) : pg.rows(kKinds == kZ);
+    const int npieces = nrows * ncg;
+    int row[kMaxItems], col[kMaxItems], cnt[kMaxItems];
     uint32_t soff[kMaxItems];
 #pragma unroll
     for (int t = 0; t < kMaxItems; ++t) {
       const int i = ptid + t * kProdThreads;
       const int j = i / ncg, c = (i - j * ncg) * 4;
-      const bool iv = i < nitems;
-      goff[t] = iv ? (int)(j * rstride) + c : 0;
+      const bool iv = i < npieces;
+      row[t] = iv ? j : 0;
+      col[t] = iv ? (kKinds == kAll ? c : j * pg.row_stride(kKinds == kZ) + c) : 0;  // one kind: the whole offset
       soff[t] = iv ? quad_offset(j, c) : 0u;
       cnt[t] = iv ? min(4, nx - c) : 0;
     }
-    auto load_items = [&](int plane, float2 (&x)[kMaxItems][4]) {
-      const bool pv = plane < a.nplanes;
-      const float2* src = a.v + (pv ? pg.base(plane) : 0);
+    auto load_plane = [&](const Items<kKinds>& w, int pl, float2 (&x)[kMaxItems][4]) {
+      const int plane = 2 * w.pair + pl;
+      const bool pv = w.more() && plane < pg.count(w.z);
+      const float2* src = a.v + (pv ? pg.base(w.z, plane) : 0);
+      const int rs = pg.row_stride(w.z), rows = pg.rows(w.z);
 #pragma unroll
-      for (int t = 0; t < kMaxItems; ++t)
+      for (int t = 0; t < kMaxItems; ++t) {
+        const float2* q = src + (kKinds == kAll ? row[t] * rs + col[t] : col[t]);
+        const int n = pv && (kKinds != kAll || row[t] < rows) ? cnt[t] : 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          x[t][u] = (pv && u < cnt[t]) ? __ldg(src + goff[t] + u) : make_float2(0.f, 0.f);
-    };
-    auto prefetch_plane = [&](int plane) {  // into L2, one 16-value row segment per thread
-      if (plane >= a.nplanes) return;
-      const int j = ptid >> 2, i = (ptid & 3) * 16;
-      if (j < nrows && i < nx) prefetch_l2(a.v + pg.base(plane) + j * rstride + i);
+        for (int u = 0; u < 4; ++u) x[t][u] = u < n ? __ldg(q + u) : make_float2(0.f, 0.f);
+      }
     };
     float2 x[kMaxItems][4];
     pdl_wait();  // v is written by the previous iteration's update
-    load_items(2 * p_first, x);  // in flight during the setup
+    Items<kKinds> w(pg, p_first, p_stride, p_end);
+    load_plane(w, 0, x);  // in flight during the setup
     int slot = 0;
-    for (int it = 0, pair = p_first; pair < npairs; pair += p_stride, ++it) {
+    for (int it = 0; w.more(); ++it) {
       const int st = it & 1;
       const uint32_t par = (uint32_t)(it >> 1) & 1u;
       if (ptid == 0)
@@ -329,16 +352,21 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
         if (ptid == 0) failed = 1;
         break;
       }
-      {  // the pair after next into L2
-        const int far = 2 * (pair + 2 * p_stride);
-        prefetch_plane(far);
-        prefetch_plane(far + 1);
+      if (kKinds != kAll) {  // the pair after next into L2, one 16-value row segment per thread
+        const int j = ptid >> 2, i = (ptid & 3) * 16;
+#pragma unroll
+        for (int pl = 0; pl < 2; ++pl) {
+          const int far = 2 * (w.pair + 2 * p_stride) + pl;
+          if (far < pg.count(w.z) && j < pg.rows(w.z) && i < nx)
+            prefetch_l2(a.v + pg.base(w.z, far) + j * pg.row_stride(w.z) + i);
+        }
       }
       uint8_t* vs = V + st * kStage;
 #pragma unroll 1
       for (int pl = 0; pl < 2; ++pl) {
         float2 y[kMaxItems][4];  // the next plane, in flight while this one is sliced
-        load_items(pl == 0 ? 2 * pair + 1 : 2 * (pair + p_stride), y);
+        if (pl == 1) w.next();
+        load_plane(w, pl ^ 1, y);
         float mx = 0.f;
 #pragma unroll
         for (int t = 0; t < kMaxItems; ++t)
@@ -349,7 +377,7 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
         if (lane == 0) red[slot][pw] = mx;
         tc::named_sync(1, kProdThreads);
 #pragma unroll
-        for (int w = 0; w < kProdWarps; ++w) mx = fmaxf(mx, red[slot][w]);
+        for (int r = 0; r < kProdWarps; ++r) mx = fmaxf(mx, red[slot][r]);
         slot ^= 1;
         const int e = plane_exponent(mx);
         if (ptid == 0) e_stage[st][pl] = e;
@@ -380,7 +408,8 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
     // ---- MMA issue ----
     const uint32_t tb = tc::smem_u32(sm);
     if (!tc::mbar_wait(&t_ready, 0u)) failed = 1;
-    for (int it = 0, pair = p_first; pair < npairs && !failed; pair += p_stride, ++it) {
+    int it = 0;
+    for (Items<kKinds> w(pg, p_first, p_stride, p_end); w.more() && !failed; w.next(), ++it) {
       const int st = it & 1;
       const uint32_t par = (uint32_t)(it >> 1) & 1u;
       if (!tc::mbar_wait(&v_full[st], par) || !tc::mbar_wait(&acc_empty[st], par ^ 1u)) {
@@ -401,7 +430,7 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
       // slice k (M = (p, x), MN-major, the planes kPlaneSlices apart), B = T
       // slices 0 .. ns - 1 - k; 16 rows (2 KiB) per K step.  The first MMA
       // (k = 0, N = 64 ns) sets every class.
-      const uint32_t t0 = tb + (kXY ? kTile : 0u);
+      const uint32_t t0 = tb + kTile, tr = kKinds == kZ ? tb : w.z ? tb + (uint32_t)a.tz_tile * kTile : t0;
       const int ns = a.nslices;
 #pragma unroll 1
       for (int k = 0; k < ns; ++k) {
@@ -410,9 +439,9 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
         for (int s = 0; s < 4; ++s)
           tc::mma_f16(d0 + (uint32_t)k * 64u,
                       tc::sw128_mn_desc(vb + (uint32_t)k * kTile + (uint32_t)s * 2048u, kPlaneSlices, 1024u),
-                      tc::sw128_desc(t0 + (uint32_t)s * 32u), idesc, (k == 0 && s == 0) ? 0u : 1u);
+                      tc::sw128_desc(tr + (uint32_t)s * 32u), idesc, (k == 0 && s == 0) ? 0u : 1u);
       }
-      if (kXY) {
+      if (kKinds != kZ && !w.z) {
         // contraction along x: A = diag(T_l, T_l) over K = (p', q), read MN-major
         // (T is symmetric) with its two 64-row blocks chosen by the start address
         // and the block stride: [T_l; 0] = (T_l, the zero tile above) and
@@ -445,34 +474,23 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
   }
 }
 
-// x and y contractions: out(y, x) = (Tx v + Ty v) as double-float pairs
-__global__ void __launch_bounds__(kWsThreads, 1) k_kin_xy_tc(KinTC a) {
-  kin_ws_body<true>(a, blockIdx.x, gridDim.x, 1 << 30);
-}
-
-// z contraction added into the pairs: out(z, x) += Tz v
-__global__ void __launch_bounds__(kWsThreads, 1) k_kin_z_tc(KinTC a) {
-  kin_ws_body<false>(a, blockIdx.x, gridDim.x, 1 << 30);
+template <int kKinds>
+__global__ void __launch_bounds__(kWsThreads, 1) k_kin_tc(KinTC a) {
+  kin_ws_body<kKinds>(a, blockIdx.x, gridDim.x, 1 << 30);
 }
 
 // Grouped launch over several problems (each with its own grid, T image and
 // vectors): CTA c works on problem work[c].x, pairs [work[c].y, work[c].z).
-__global__ void __launch_bounds__(kWsThreads, 1) k_kin_xy_tc_group(const KinTC* __restrict__ probs,
-                                                                    const int4* __restrict__ work) {
+template <int kKinds>
+__global__ void __launch_bounds__(kWsThreads, 1) k_kin_tc_group(const KinTC* __restrict__ probs,
+                                                                 const int4* __restrict__ work) {
   const int4 w = work[blockIdx.x];
   const KinTC a = probs[w.x];
-  kin_ws_body<true>(a, w.y, 1, w.z);
-}
-__global__ void __launch_bounds__(kWsThreads, 1) k_kin_z_tc_group(const KinTC* __restrict__ probs,
-                                                                   const int4* __restrict__ work) {
-  const int4 w = work[blockIdx.x];
-  const KinTC a = probs[w.x];
-  kin_ws_body<false>(a, w.y, 1, w.z);
+  kin_ws_body<kKinds>(a, w.y, 1, w.z);
 }
 
-constexpr size_t kSmemXY = 1024 + (kTS + 2) * kTile + kStages * kStage;
-constexpr size_t kSmemZ = 1024 + kTS * kTile + kStages * kStage;
-static_assert(kSmemXY + 512 <= 227 * 1024, "x/y T tiles and stages must fit in one CTA's shared memory");
+constexpr size_t smem_bytes(int kinds) { return 1024 + (size_t)t_tiles(kinds) * kTile + kStages * kStage; }
+static_assert(smem_bytes(kAll) + 512 <= 227 * 1024, "the T tiles and the stages must fit in one CTA's shared memory");
 static_assert(kStages * kAccCols <= 512, "the accumulator stages must fit in tensor memory");
 
 int sm_count() {
@@ -540,84 +558,106 @@ void kinetic_slices_f32(const std::vector<double>& T, int n, std::vector<float>*
 bool kinetic_tc_supported(const Tables& t) { return t.nx <= 64 && t.ny <= 64 && t.nz <= 64 && t.tx == t.ty; }
 
 namespace {
-// the kernel arguments of one problem's x/y (xy = true) or z contraction of v
-// (fin_count > 0: the x/y launch finishes a deferred beta of that many block totals)
-KinTC kin_tc_args(bsl_handle* h, const float2* v, bool xy, int fin_count) {
+// the kernel arguments of one problem's contractions of v (fin_count > 0: the
+// launch finishes a deferred beta of that many block totals)
+KinTC kin_tc_args(bsl_handle* h, const float2* v, int kinds, int fin_count) {
   const Tables& t = h->t;
   DeviceState& d = h->d;
   KinTC a{};
   a.v = v;
-  a.out = reinterpret_cast<float2*>(d.ukin);
+  a.out_xy = reinterpret_cast<float2*>(d.ukin);
+  a.out_z = kinds == kAll ? d.ukin_z : a.out_xy;
   a.nx = t.nx;
   a.ny = t.ny;
   a.nz = t.nz;
+  a.nn = t.nn;
   a.status = d.status;
   a.nslices = h->kin_slices;
-  if (xy) {
-    a.timage = reinterpret_cast<const uint4*>(d.kxy_slices);
-    a.timage16 = (int)((kTS + 2) * kTile / 16);
-    a.e_t = d.e_txy;
-    a.nplanes = t.nz * t.nn;
-    if (fin_count > 0) {
-      a.fin_partials = d.partials;
-      a.scalars = d.scalars;
-      a.hist = d.hist;
-      a.jdev = d.jdev;
-      a.fin_count = fin_count;
-      a.hist_stride = d.hist_cap;
-    }
-  } else {
-    a.timage = reinterpret_cast<const uint4*>(d.kz_slices);
-    a.timage16 = (int)(kTS * kTile / 16);
-    a.e_t = d.e_tz;
-    a.nplanes = t.ny * t.nn;
+  const int tile16 = (int)(kTile / 16);
+  a.timage = reinterpret_cast<const uint4*>(d.kin_slices) + (kinds == kZ ? d.kin_tz_tile * tile16 : 0);
+  a.timage16 = kinds == kAll ? d.kin_image16 : t_tiles(kinds) * tile16;
+  a.tz_tile = d.kin_tz_tile;
+  a.e_txy = d.e_txy;
+  a.e_tz = d.e_tz;
+  if (fin_count > 0) {
+    a.fin_partials = d.partials;
+    a.scalars = d.scalars;
+    a.hist = d.hist;
+    a.jdev = d.jdev;
+    a.fin_count = fin_count;
+    a.hist_stride = d.hist_cap;
   }
   return a;
 }
+
+long long pairs_of(const Tables& t, int kinds) {
+  return ((long long)(kinds == kXY ? t.nz : kinds == kZ ? t.ny : std::max(t.nz, t.ny)) * t.nn + 1) / 2;
+}
+
+template <int kKinds>
+int launch_kinds(bsl_handle* h, const float2* v, cudaStream_t s) {
+  cudaFuncSetAttribute(k_kin_tc<kKinds>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(kKinds));
+  const KinTC a = kin_tc_args(h, v, kKinds, kKinds != kZ && h->defer_reductions ? deferred_beta_count(h) : 0);
+  BSL_CUDA(launch_pdl(k_kin_tc<kKinds>, dim3((unsigned)std::min<long long>(pairs_of(h->t, kKinds), sm_count())),
+                      dim3(kWsThreads), smem_bytes(kKinds), s, a));
+  BSL_CUDA(cudaGetLastError());
+  return BSL_OK;
+}
 }  // namespace
+
+// The shared-memory image of both matrices: Z T0 .. T3 Z of x and y, and the
+// slices of Tz after it unless Tz is the same matrix (*tz_tile: its first tile).
+void kinetic_tc_image(const Tables& t, std::vector<uint16_t>* image, int* tz_tile, int* e_txy, int* e_tz) {
+  kinetic_smem_image(t.tx, t.nx, true, image, e_txy);
+  if (t.tz == t.tx) {
+    *tz_tile = 1;
+    *e_tz = *e_txy;
+    return;
+  }
+  *tz_tile = kTS + 2;
+  std::vector<uint16_t> z;
+  kinetic_smem_image(t.tz, t.nz, false, &z, e_tz);
+  image->insert(image->end(), z.begin(), z.end());
+}
 
 size_t kin_group_arg_size() { return sizeof(KinTC); }
 
 // the plane pairs of one problem's x/y or z contraction (the work units)
-long long kin_tc_pairs(const bsl_handle* h, bool xy) {
-  const Tables& t = h->t;
-  return ((long long)(xy ? t.nz : t.ny) * t.nn + 1) / 2;
-}
+long long kin_tc_pairs(const bsl_handle* h, bool xy) { return pairs_of(h->t, xy ? kXY : kZ); }
 
 // fill args[b] (kin_group_arg_size() bytes each) for the problems' vectors v[b]
 void kin_tc_group_args(bsl_handle** hs, int n, const float2* const* v, bool xy, const int* fin_counts, void* args) {
   KinTC* a = static_cast<KinTC*>(args);
-  for (int b = 0; b < n; ++b) a[b] = kin_tc_args(hs[b], v[b], xy, fin_counts ? fin_counts[b] : 0);
+  for (int b = 0; b < n; ++b) a[b] = kin_tc_args(hs[b], v[b], xy ? kXY : kZ, fin_counts ? fin_counts[b] : 0);
 }
 
 int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nctas, cudaStream_t s) {
-  const size_t smem = xy ? kSmemXY : kSmemZ;
-  if (xy) {
-    cudaFuncSetAttribute(k_kin_xy_tc_group, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BSL_CUDA(launch_pdl(k_kin_xy_tc_group, dim3(nctas), dim3(kWsThreads), smem, s,
-                        static_cast<const KinTC*>(d_args), d_work));
-  } else {
-    cudaFuncSetAttribute(k_kin_z_tc_group, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BSL_CUDA(launch_pdl(k_kin_z_tc_group, dim3(nctas), dim3(kWsThreads), smem, s,
-                        static_cast<const KinTC*>(d_args), d_work));
-  }
+  const auto kernel = xy ? k_kin_tc_group<kXY> : k_kin_tc_group<kZ>;
+  const size_t smem = smem_bytes(xy ? kXY : kZ);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  BSL_CUDA(launch_pdl(kernel, dim3(nctas), dim3(kWsThreads), smem, s, static_cast<const KinTC*>(d_args), d_work));
   return BSL_OK;
+}
+
+// One launch up to 800,000 coefficients.  There a launch of either kind is a few
+// plane pairs a CTA, so that setting up a CTA (tensor memory, the T tiles, the
+// zeroed stages) and draining it are most of its 10-22 us, and one launch pays
+// for them once; the z part, 8 bytes a coefficient more for the apply to read,
+// stays in L2.  An iteration in one launch against two: 20^3 with 21 functions
+// 34.2 against 39.3 us, 24^3 with 10 22.9 against 27.6, 27^3 with 21 36.7
+// against 42.2, 33^3 with 15 35.1 against 38.7, with 21 45.1 against 50.5.
+// Beyond, the z launch's setup is hidden behind the x/y launch's tail and the
+// added bytes are not: 41^3 with 21 62.2 against 58.5 us, 54^3 113 against 88.
+bool kin_tc_one_launch(const bsl_handle* h) {
+  return h->t.npts * h->t.nn <= 800000;
 }
 
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s) {
-  cudaFuncSetAttribute(k_kin_xy_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemXY);
-  const KinTC a = kin_tc_args(h, v, true, h->defer_reductions ? deferred_beta_count(h) : 0);
-  BSL_CUDA(launch_pdl(k_kin_xy_tc, dim3(std::min((a.nplanes + 1) / 2, sm_count())), dim3(kWsThreads), kSmemXY, s, a));
-  BSL_CUDA(cudaGetLastError());
-  return BSL_OK;
+  return kin_tc_one_launch(h) ? launch_kinds<kAll>(h, v, s) : launch_kinds<kXY>(h, v, s);
 }
 
 int launch_kin_z_tc(bsl_handle* h, const float2* v, cudaStream_t s) {
-  cudaFuncSetAttribute(k_kin_z_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemZ);
-  const KinTC a = kin_tc_args(h, v, false, 0);
-  BSL_CUDA(launch_pdl(k_kin_z_tc, dim3(std::min((a.nplanes + 1) / 2, sm_count())), dim3(kWsThreads), kSmemZ, s, a));
-  BSL_CUDA(cudaGetLastError());
-  return BSL_OK;
+  return kin_tc_one_launch(h) ? BSL_OK : launch_kinds<kZ>(h, v, s);
 }
 
 }  // namespace bsl

@@ -357,6 +357,7 @@ int build_grouped(bsl_handle** hs, int n, GroupedBatch* g) {
       double* Vd = p ? d.rvec : d.vec;
       double* Rd = p ? d.vec : d.rvec;
       StreamArgs a = vstream_args(h, Vd, Rd);
+      a.ukin_z = nullptr;        // the grouped kinetic adds z in a launch of its own
       a.red_count = ctas[2][b];  // the light apply's blocks: alpha's block totals
       std::memcpy(host.data() + off_args[2][p] + sz[2] * b, &a, sizeof(a));
       a.red_count = ctas[3][b];  // the fused update's CTAs: beta's block totals
@@ -854,8 +855,9 @@ int bsl_stage_times(bsl_handle* h, int iters, double* ms, const char** names) {
 
 int bsl_launches_per_iteration(const bsl_handle* h) {
   if (!h) return -1;
-  // kinetic in one launch: small grids in mixed precision, FP64 without the tensor cores
-  const bool one = h->precision == BSL_PREC_MIXED ? h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)
+  // kinetic in one launch: small problems in mixed precision, FP64 without the tensor cores
+  const bool one = h->precision == BSL_PREC_MIXED ? h->kinetic_engine == BSL_KIN_TENSOR &&
+                                                        (kin_small_supported(h) || kin_tc_one_launch(h))
                                                   : !kin_f64_tensor(h);
   return one ? 3 : 4;
 }

@@ -327,6 +327,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
           for (int u = 0; u < kGroup; ++u)
             if (s0 + u < NN) {
               uk[u] = A.ukin[(s0 + u) * npts + p];
+              if (A.ukin_z) uk[u] = df_add_fast(uk[u], A.ukin_z[(s0 + u) * npts + p]);
               rr[u] = Rp[(s0 + u) * npts + p];
             }
 #pragma unroll
@@ -345,7 +346,8 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       } else {
 #pragma unroll
         for (int s = 0; s < NN; ++s) {
-          const float2 uk = A.ukin[s * npts + p];
+          float2 uk = A.ukin[s * npts + p];
+          if (A.ukin_z) uk = df_add_fast(uk, A.ukin_z[s * npts + p]);
           const float a = fmaf(__ldg(A.rot_hi + s), vv[s], va[s]);
           float hi, e;
           two_sum(uk.x, a, hi, e);
@@ -425,7 +427,7 @@ __global__ void __launch_bounds__(kTilePts, vstream_min_ctas(NN)) k_vstream(cons
 // is block `index` of the `count` that reduce alpha.
 constexpr int kLightThreads = 256;
 constexpr int kLightGroup = 7;
-template <int NN, int kGroup>
+template <int NN, int kGroup, bool kApart = false>
 __device__ __forceinline__ void light_body(const StreamArgs& A, long long p, unsigned int index,
                                            unsigned int count) {
   const int tid = threadIdx.x;
@@ -447,6 +449,7 @@ __device__ __forceinline__ void light_body(const StreamArgs& A, long long p, uns
           const long long i = (s0 + u) * npts + p;
           vx[u] = Vp[i];
           uk[u] = A.ukin[i];
+          if (kApart) uk[u] = df_add_fast(uk[u], A.ukin_z[i]);  // the z part is kept apart
           rr[u] = Rp[i];
           va[u] = A.vprod[i];
         }
@@ -473,9 +476,9 @@ __device__ __forceinline__ void light_body(const StreamArgs& A, long long p, uns
   }
 }
 
-template <int NN, int kGroup>
+template <int NN, int kGroup, bool kApart = false>
 __global__ void __launch_bounds__(kLightThreads) k_vapply_light(const StreamArgs A) {
-  light_body<NN, kGroup>(A, (long long)blockIdx.x * kLightThreads + threadIdx.x, blockIdx.x, gridDim.x);
+  light_body<NN, kGroup, kApart>(A, (long long)blockIdx.x * kLightThreads + threadIdx.x, blockIdx.x, gridDim.x);
 }
 
 // Grouped launches over problems with blocks of 15 or 21 functions (the fused
@@ -848,14 +851,17 @@ int launch_vapply_light(const StreamArgs& a, int nn, cudaStream_t s) {
   const bool one = grid <= sms;
   cudaError_t e;
   if (nn == 10)
-    e = launch_pdl(one ? k_vapply_light<10, 10> : k_vapply_light<10, kLightGroup>, dim3((unsigned)grid),
-                   dim3(kLightThreads), 0, s, a);
+    e = launch_pdl(one ? (a.ukin_z ? k_vapply_light<10, 10, true> : k_vapply_light<10, 10>)
+                       : (a.ukin_z ? k_vapply_light<10, kLightGroup, true> : k_vapply_light<10, kLightGroup>),
+                   dim3((unsigned)grid), dim3(kLightThreads), 0, s, a);
   else if (nn == 15)
-    e = launch_pdl(one ? k_vapply_light<15, 15> : k_vapply_light<15, kLightGroup>, dim3((unsigned)grid),
-                   dim3(kLightThreads), 0, s, a);
+    e = launch_pdl(one ? (a.ukin_z ? k_vapply_light<15, 15, true> : k_vapply_light<15, 15>)
+                       : (a.ukin_z ? k_vapply_light<15, kLightGroup, true> : k_vapply_light<15, kLightGroup>),
+                   dim3((unsigned)grid), dim3(kLightThreads), 0, s, a);
   else if (nn == 21)
-    e = launch_pdl(one ? k_vapply_light<21, 21> : k_vapply_light<21, kLightGroup>, dim3((unsigned)grid),
-                   dim3(kLightThreads), 0, s, a);
+    e = launch_pdl(one ? (a.ukin_z ? k_vapply_light<21, 21, true> : k_vapply_light<21, 21>)
+                       : (a.ukin_z ? k_vapply_light<21, kLightGroup, true> : k_vapply_light<21, kLightGroup>),
+                   dim3((unsigned)grid), dim3(kLightThreads), 0, s, a);
   else
     return fail(BSL_ERR_UNSUPPORTED, "light apply: unsupported block size");
   return e == cudaSuccess ? BSL_OK : cuda_fail(e, "light apply launch");

@@ -104,14 +104,17 @@ def test_fp64_hv_after_a_reported_time_out(bsl, tmp_path):
         h.close()
 
 
-# one launch up to 16 points: smallest grids, planes of a full and of a broken warp
-# count, unequal z, the last size of the range and the first beyond it
+# one launch: up to 16 points on the CUDA cores (smallest grids, planes of a full and of
+# a broken warp count, unequal z, the last size of the range and the first beyond it), up
+# to 800,000 coefficients on the tensor cores (z shorter and longer than y, more plane
+# pairs than CTAs, the last cube of the range); the first size with two launches
 @pytest.mark.parametrize("n,nz,l_max,sym", [(4, 4, 4, "Even"), (5, 16, 5, "Odd"), (11, 6, 3, "Odd"), (7, 9, 3, "All"),
                                             (16, 16, 4, "Even"), (16, 15, 5, "Odd"), (17, 16, 4, "Even"),
-                                            (16, 17, 3, "Odd")])
+                                            (16, 17, 3, "Odd"), (20, 33, 5, "Odd"), (33, 20, 4, "Even"),
+                                            (21, 64, 3, "Odd"), (33, 33, 5, "Odd"), (34, 33, 5, "Odd")])
 def test_small_grid_kinetic(bsl, tmp_path, n, nz, l_max, sym):
     """Mixed H v with the one-launch kinetic against the FP64 path, and against
-    the two-launch kinetic: with three slices of v and T, and with four, it
+    the tensor-core kinetic of three slices: with four slices of v and T it
     differs from FP64 by those slices' truncation only."""
     import ctypes as C
     h = bsl.Hamiltonian(write_case(str(tmp_path), (n, n, nz), l_max, sym), CALC, precision="fp64")
@@ -120,13 +123,14 @@ def test_small_grid_kinetic(bsl, tmp_path, n, nz, l_max, sym):
         ref, u, u3 = np.zeros_like(v), np.zeros_like(v), np.zeros_like(v)
         h.hv(v, ref)
         h.set_precision("mixed")
-        assert bsl.lib().bsl_launches_per_iteration(C.c_void_p(h.handle.value)) == (3 if max(n, nz) <= 16 else 4)
+        hp = C.c_void_p(h.handle.value)
+        assert bsl.lib().bsl_launches_per_iteration(hp) == (3 if bsl.lib().bsl_packed_size(hp) <= 800000 else 4)
         h.hv(v, u)
         # FP32 potential: (nn + 3) roundings of 2^-24 at |V| <= 18 |v|; the kinetic's
         # slices leave 2^-33 of max |T| max |v| per direction
         tol = np.max(np.abs(v)) * (40 * 2.0 ** -24 * 18.0 + 8 * 2.0 ** -33 * kinetic_scale((n, n, nz)))
         assert np.max(np.abs(u - ref)) <= tol
-        h.set_kinetic_slices(3)  # two launches
+        h.set_kinetic_slices(3)  # the tensor-core kernel
         h.hv(v, u3)
         # the dropped class: four products a_k b_l of |a|, |b| <= 256, n terms each
         drop = 4 * 256 * 256 * 2.0 ** (-16 - 27) * 4 * kinetic_scale((n, n, nz)) * max(n, nz) * np.max(np.abs(v))
