@@ -443,10 +443,11 @@ int hv_prep(const bsl_hv_params* params, const Cage* cage, bsl_handle** out) {
     if ((rc = upload(&d.tx_slices32, sf, "Tx"))) return bail(rc);
     kinetic_slices_f32(t.tz, t.nz, &sf);
     if ((rc = upload(&d.tz_slices32, sf, "Tz"))) return bail(rc);
-    kinetic_smem_image64(t.tx, t.nx, true, &sl, &d.e_txy64);
-    if ((rc = upload(&d.kxy_slices64, sl, "Tx"))) return bail(rc);
-    kinetic_smem_image64(t.tz, t.nz, false, &sl, &d.e_tz64);
-    if ((rc = upload(&d.kz_slices64, sl, "Tz"))) return bail(rc);
+    std::vector<uint16_t> slz;
+    if (kinetic_smem_image64(t.tx, t.nx, &sl, &d.e_txy64) &&
+        kinetic_smem_image64(t.tz, t.nz, &slz, &d.e_tz64) &&
+        ((rc = upload(&d.kxy_slices64, sl, "Tx")) || (rc = upload(&d.kz_slices64, slz, "Tz"))))
+      return bail(rc);
     h->kinetic_engine = BSL_KIN_TENSOR;
   }
   if ((rc = upload(&d.rot, t.rot, "rotor"))) return bail(rc);

@@ -101,7 +101,7 @@ struct DeviceState {
   int kin_image16 = 0, kin_tz_tile = 0, e_txy = 0, e_tz = 0;
   float2* ukin_z = nullptr;        // one-launch tensor-core kinetic: the z part (x/y in ukin)
   float *tx_slices32 = nullptr, *tz_slices32 = nullptr;  // the slices as FP32 integers (bsl_small.cu)
-  // the same for the FP64 path: seven slices (bsl_kinetic_tc64.cu)
+  // the same for the FP64 path: eight slices (bsl_kinetic_tc64.cu); null where it does not take T
   uint16_t *kxy_slices64 = nullptr, *kz_slices64 = nullptr;
   int e_txy64 = 0, e_tz64 = 0;
   int kin_grid_xy = 0, kin_grid_z = 0;  // persistent grid sizes
@@ -241,8 +241,7 @@ void kinetic_slices_f32(const std::vector<double>& T, int n, std::vector<float>*
 bool kin_small_supported(const bsl_handle* h);
 int launch_kin_small(bsl_handle* h, const float2* v, int fin_count, cudaStream_t s);
 // FP64 kinetic on the tensor cores (bsl_kinetic_tc64.cu): FP64 v, FP64 output
-void kinetic_smem_image64(const std::vector<double>& T, int n, bool with_zero_tiles, std::vector<uint16_t>* image,
-                          int* e_t);
+bool kinetic_smem_image64(const std::vector<double>& T, int n, std::vector<uint16_t>* image, int* e_t);
 int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s);
 bool kin_f64_tensor(const bsl_handle* h);
 void kinetic_tc_image(const Tables& t, std::vector<uint16_t>* image, int* tz_tile, int* e_txy, int* e_tz);

@@ -5,32 +5,47 @@
 // Hv-calculators/linRotor/cartSphBasis/HvCalc/linRotCartSphHvRoutines.cpp:1807-1969.
 //
 // The contractions of bsl_kinetic_tc.cu (the same plane pairs, tiles, swizzle
-// and accumulator layout) for FP64 vectors: v and T are cut into seven 9-bit
-// integer slices instead of four (after Ozaki, Ogita, Oishi and Rump, Numer.
-// Algorithms 59, 2012), 62 bits below the plane's and the matrix's largest
-// element, and the 28 products of the classes k + l <= 6 are kept.  What is left
-// out is 2^-62 of max|v| max|T| per term, below the rounding of an FP64 dot
-// product (2^-53 of its partial sums): see test_kinetic_f64_slicing.py.
-// The class sums 0-3 are integers below 2^24 and exact; the sums of classes 4-6
-// could pass 2^24 only for a v that follows the signs of T's low slices, and
-// one unit there is 2^-52 and less of the FP64 unit.  The classes are put
-// together in 64-bit integers and rounded once to FP64.
+// and accumulator layout) for FP64 vectors: every line of v that is contracted (a
+// column of the plane along y or z, a row along x) and T are cut into eight 9-bit
+// integer slices (after Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59,
+// 2012) and the 36 products of the classes k + l <= 7 are kept.
+//
+// What that leaves out, of max |T| times the line's largest |v|, for an element of
+// the result:
+//   * an element of v is cut 71 bits below its own line's largest element (an
+//     exponent per line, so that a small line keeps its bits beside a large one);
+//     T is cut there too, which is exact down to 2^-18 max |T| (the smallest
+//     element of a 64-point axis is 2^-12.7 of the largest);
+//   * the classes from 8 on: 2^-69 root mean square for 64 terms of digits without
+//     a pattern, at most 2^-63;
+//   * the class sums 0-6 are integers below 2^24 and exact (kinetic_smem_image64
+//     refuses a T whose slices could pass that), class 7 is rounded at 2^-71;
+//   * the classes are put together as integers and rounded once.
+// The sum of |T v| along the line is at least 2^-12.7 of the same product, so this
+// stays below one FP64 rounding (2^-53) of that sum, and below a dot product's
+// n 2^-53 even at its largest: every element is held to its own terms as in FP64,
+// whatever the range of v (the tail of a bound state, a column of 1e-20 beside
+// one of 1): test_kinetic_f64_lines.py, test_gpu_kinetic_f64.py.  A line with an
+// infinity or a NaN is formed by the plain sums.
 //
 // Why: the FP64 pipe executes 2 lanes a clock and SM, so 3 x 54 multiply-adds
-// per coefficient take 0.85 ms at 54^3 and 21 functions; the 28 slice products
-// are 18 us of tensor-core time.  Measured at 54^3, 21
-// functions, x/y and z: 70 and 57 us against 656 and 337 us, and 28 and 24 us
-// against 49 and 29 us at 27^3; bound by the shared-memory reads of the MMA
-// operands (x/y) and the FP64 conversions and read-modify-write of the epilogue
-// (z).
+// per coefficient take 0.85 ms at 54^3 and 21 functions.  Measured there, x/y and
+// z: 104 and 57 us against 656 and 337 us of plain sums in two launches; 38 and
+// 23 us at 27^3.  An item (a plane pair and direction) takes its slicing (11,000
+// clocks, integer pipe) and its MMAs (8,000) in turn, since the eight slices leave
+// room for one stage; the epilogue (13,000, FP64 additions and the
+// read-modify-write) runs beside them.
 //
 // Pipeline: as there, 8 epilogue warps, 8 producer warps and one MMA thread, but
-// with one shared-memory stage (112 KiB) and one accumulator (448 columns): the
-// producers slice the next pair while the epilogue reads the finished one.
+// with one shared-memory stage (128 KiB).  The accumulator has two parts, for
+// half of T's rows each, so that the epilogue reads one while the other's MMAs
+// run.  The x/y kernel takes a pair of planes as two items, along y and along x,
+// since the lines, and so the slices, differ.
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "bsl_device.cuh"
@@ -40,53 +55,70 @@
 namespace bsl {
 namespace {
 
-constexpr int kS = 7;                           // slices of v and of T
+constexpr int kS = 8;                           // slices of v and of T
 constexpr uint32_t kTile = 64 * 128;            // 64 rows x 64 FP16, one 128-byte swizzled row each
-constexpr uint32_t kPlane = kS * kTile;         // the slices of one plane
-constexpr uint32_t kAccCols = kS * 64;          // classes 0..6
+constexpr uint32_t kPair = 2 * kTile;           // one slice of a plane pair: 128 rows
+constexpr uint32_t kHalfTile = kTile / 2;       // half of the rows of a slice of T
+constexpr uint32_t kAccCols = kS * 32;          // classes 0..7 of half of the columns
 constexpr int kEpiWarps = 8, kProdWarps = 8, kMmaWarp = kEpiWarps + kProdWarps;
 constexpr int kThreads64 = (kMmaWarp + 1) * 32;
 constexpr int kProdThreads = kProdWarps * 32, kEpiThreads = kEpiWarps * 32;
-constexpr int kMaxItems = 64 * 16 / kProdThreads;  // (row, 4-column group) items per producer thread
-constexpr int kNonFinite = 1 << 20;                // plane exponent of a plane with an infinity or a NaN
+constexpr int kMaxItems = 64 * 16 / kProdThreads;  // (row, 4-column group) pieces per producer thread
+constexpr int kNonFinite = 1 << 20;                // exponent of a line with an infinity or a NaN
 
 struct Kin64 {
   const uint4* timage;  // the T tiles as laid out in shared memory
   int timage16;
   int e_t;
+  const double* t;      // T, for the lines that are not finite
   const double* v;
   double* out;
   int nx, ny, nz, nplanes;
   int* status;
 };
 
-// 512^0 + ... + 512^6, times 256: added to the 62-bit fixed-point value, every
-// 9-bit digit d stands for d - 256
-constexpr unsigned long long kBias = 256ull * ((1ull << 54) + (1ull << 45) + (1ull << 36) + (1ull << 27) +
-                                               (1ull << 18) + (1ull << 9) + 1ull);
+// 36 bits of a fixed-point value are four 9-bit digits; 256 in every digit makes
+// each digit d stand for d - 256
+constexpr long long kBias36 = 256ll * ((1ll << 27) + (1ll << 18) + (1ll << 9) + 1ll);
+constexpr unsigned long long kMask36 = (1ull << 36) - 1;
+
+// T's rows (the results' columns) are taken in two halves, of a multiple of 4 and
+// at most 32 rows the first, so that the accumulator has two parts
+__host__ __device__ __forceinline__ int half_rows(int n) { return (n + 7) / 8 * 4; }
 
 __device__ __forceinline__ uint32_t quad_offset64(int r, int k) {
   return (uint32_t)(r * 128 + (((k >> 3) ^ (r & 7)) << 4) + ((k & 7) << 1));
 }
 
-// v 2^(62 - e) + kBias for |v| < 2^e (truncated below 2^-62 of 2^e)
-__device__ __forceinline__ unsigned long long fixed_point(double v, int e) {
-  const long long b = __double_as_longlong(v);
-  const int ev = (int)(((unsigned long long)b >> 52) & 0x7ff);
-  unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (1ull << 52);
-  const int sh = ev - 1013 - e;  // at most 9
-  m = sh >= 0 ? m << min(sh, 9) : m >> min(-sh, 63);
-  if (ev == 0) m = 0;
-  return kBias + (b < 0 ? 0ull - m : m);
+// e of a line whose largest |v| has the upper word hi: |v| < 2^e
+__device__ __forceinline__ int line_exponent(unsigned int hi) {
+  const int ev = (int)(hi >> 20);
+  return ev == 0x7ff ? kNonFinite : max(ev, 1) - 1022;
 }
 
-// digits k of two values as FP16 integers in [-256, 256]
+// v 2^(71 - e), truncated, for |v| < 2^e of a line whose largest exponent field
+// (at least 1) is top, as eight biased digits, four in each of hi and lo
+struct Digits {
+  unsigned long long hi, lo;
+};
+__device__ __forceinline__ Digits digits_of(double v, int top) {
+  const long long b = __double_as_longlong(v);
+  const int ev = (int)(((unsigned long long)b >> 52) & 0x7ff);
+  unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+  if (ev) m |= 1ull << 52;
+  const int d = top - max(ev, 1);  // v 2^(71 - e) = m 2^(18 - d)
+  const long long mh = (long long)(m >> min(18 + d, 63));
+  const long long ml = (long long)((d <= 18 ? m << (18 - d) : m >> min(d - 18, 63)) & kMask36);
+  const long long s = kBias36 + (b < 0 ? -ml : ml);
+  return Digits{(unsigned long long)(kBias36 + (b < 0 ? -mh : mh) + (s >> 36)), (unsigned long long)s & kMask36};
+}
+
+// digit k of two 36-bit groups as FP16 integers in [-256, 256] (the top digit reaches 512 before the bias)
 template <int kDigit>
 __device__ __forceinline__ uint32_t slice2(unsigned long long a, unsigned long long b) {
-  const uint32_t mask = kDigit == kS - 1 ? 0x3ffu : 0x1ffu;  // the top digit reaches 512
-  const uint32_t x = (uint32_t)(a >> (9 * kDigit)) & mask, y = (uint32_t)(b >> (9 * kDigit)) & mask;
+  constexpr uint32_t mask = kDigit == 3 ? 0x03ff03ffu : 0x01ff01ffu;
   // 0x6400 + d is 1024 + d in FP16 for d < 1024
-  uint32_t r = (x | (y << 16)) + 0x64006400u;
+  const uint32_t r = (__byte_perm((uint32_t)(a >> (9 * kDigit)), (uint32_t)(b >> (9 * kDigit)), 0x5410) & mask) | 0x64006400u;
   const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&r), __floats2half2_rn(1280.f, 1280.f));
   return *reinterpret_cast<const uint32_t*>(&h);
 }
@@ -98,74 +130,111 @@ struct Planes64 {
     if (kXY) return (long long)plane * nx * ny;
     return (long long)(plane / ny) * nz * nx * ny + (long long)(plane % ny) * nx;
   }
-  __device__ __forceinline__ long long row_stride() const { return kXY ? (long long)nx : (long long)nx * ny; }
+  __device__ __forceinline__ int row_stride() const { return kXY ? nx : nx * ny; }
   __device__ __forceinline__ int rows() const { return kXY ? ny : nz; }
 };
 
-// x 2^s rounded to FP64, |x| < 2^62, on the integer pipe (a conversion and a
-// product on the FP64 pipe would take 16 clocks of the SM each)
-__device__ __forceinline__ double scaled(long long x, int s) {
-  if (x == 0) return 0.0;
-  const unsigned long long m = (unsigned long long)(x < 0 ? -x : x);
-  const int lz = __clzll((long long)m);  // at least 2
-  // the leading 53 bits, rounded to nearest (ties up), the leading one at bit 52
-  const unsigned long long r = ((m << (lz - 1)) + 0x200ull) >> 10;
-  const int e = s + 1085 - lz;  // biased exponent less 1: r's leading one adds 1 to it
-  const unsigned long long sign = (unsigned long long)x & 0x8000000000000000ull;
-  if ((unsigned int)e < 2045u) return __longlong_as_double((long long)(sign | (((unsigned long long)e << 52) + r)));
-  // out of the normal range
-  return ldexp(__longlong_as_double((long long)(sign | ((1074ull << 52) + r))), e - 1074);
+// The CTA's items: one per plane pair first, first + stride, ..., or two (along y,
+// then along x) for x/y.
+template <bool kXY>
+struct Items64 {
+  int pair, stride, end;
+  bool along_x = false;
+  __device__ __forceinline__ bool more() const { return pair < end; }
+  __device__ __forceinline__ void next() {
+    if (kXY) along_x = !along_x;
+    if (!along_x) pair += stride;
+  }
+};
+
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+
+// What a thread's line scales by: class 3's unit 2^s as 2^b 2^rest, rest 0 unless
+// the products with 2^b could leave the normal range, and -(3 2^51 + 3 2^23) 2^b.
+struct LineScale {
+  int b, rest;
+  double unit, shift;
+  __device__ __forceinline__ explicit LineScale(int s) : b(min(max(s, -900), 900)) {
+    rest = s - b;
+    unit = pow2(b);
+    shift = __longlong_as_double((long long)(1023 + b + 52) << 52 | 0x8008000001800000ll);
+  }
+};
+
+// (hi + lo 2^-28) 2^b rounded to nearest: hi and lo placed in the mantissas of
+// 3 2^51 + hi and 3 2^23 + lo 2^-28 and added with one rounding.  (The same on the
+// integer pipe, about 40 operations, is no faster: 386 against 367 us an iteration.)
+__device__ __forceinline__ double rounded(long long hi, long long lo, const LineScale& q) {
+  const double h = __longlong_as_double(hi + (0x4338ll << 48)), l = __longlong_as_double(lo + (0x4178ll << 48));
+  return fma(l, q.unit, fma(h, q.unit, q.shift));
 }
 
-// 4 consecutive columns of the seven classes as FP64 values times 2^s
-__device__ __forceinline__ void combine4(uint32_t taddr, int s, double (&out)[4]) {
+// 4 consecutive columns of the eight classes as FP64 values.  Classes 0-3 and 4-7
+// are put together as 64-bit integers, the second in units of 2^-28 of class 3's
+// (class 7 rounded there: 2^-71 of 2^(e + e_t)), and rounded once.
+__device__ __forceinline__ void combine4(uint32_t taddr, const LineScale& q, double (&out)[4]) {
   float c[kS][4];
 #pragma unroll
-  for (int k = 0; k < kS; ++k) tc::tmem_ld4_nowait(taddr + 64u * k, c[k]);
+  for (int k = 0; k < kS; ++k) tc::tmem_ld4_nowait(taddr + 32u * k, c[k]);
   tc::tmem_wait_ld();
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    // units of 2^-41 of class 0's: below 2^62, and 2^-57 of 2^(e + e_t)
-    const float low = __fmaf_rn(c[6][u], 0x1p-18f, __fmaf_rn(c[5][u], 0x1p-9f, c[4][u]));
-    const int h01 = __float2int_rn(c[0][u]) * 512 + __float2int_rn(c[1][u]);
-    const long long h23 = (long long)__float2int_rn(c[2][u]) * 512 + __float2int_rn(c[3][u]);
-    const long long x = (((long long)h01 << 18) + h23) * 16384 + __float2int_rn(__fmul_rn(low, 32.f));
-    out[u] = scaled(x, s);
+    const int c12 = __float2int_rn(c[1][u]) * 512 + __float2int_rn(c[2][u]);
+    const int c67 = __float2int_rn(__fmaf_rn(c[7][u], 0x1p-8f, __fadd_rn(c[6][u], c[6][u])));
+    const long long hi = ((long long)__float2int_rn(c[0][u]) << 27) + ((long long)c12 << 9) + __float2int_rn(c[3][u]);
+    const long long lo = ((long long)__float2int_rn(c[4][u]) << 19) + ((long long)__float2int_rn(c[5][u]) << 10) + c67;
+    out[u] = rounded(hi, lo, q);
   }
+  for (int rest = q.rest; rest != 0;) {
+    const int k = min(max(rest, -1000), 1000);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) out[u] *= pow2(k);
+    rest -= k;
+  }
+}
+
+// one element by the plain sum (a line with an infinity or a NaN)
+__device__ __forceinline__ double plain_sum(const double* trow, const double* v, int stride, int n) {
+  double acc = 0.0;
+#pragma unroll 1
+  for (int q = 0; q < n; ++q) acc += __ldg(trow + q) * __ldg(v + (long long)q * stride);
+  return acc;
 }
 
 template <bool kXY>
 __device__ __forceinline__ void kin64_body(const Kin64& a) {
   extern __shared__ uint8_t smraw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
-  // T tiles: x/y as Z T0 .. T6 Z (Z = zero tile), z as T0 .. T6; then the v stage
-  constexpr int kTTiles = kXY ? kS + 2 : kS;
-  uint8_t* V = sm + kTTiles * kTile;
-  __shared__ uint64_t v_full, v_empty, acc_full, acc_empty, e_full, stage_zeroed, t_ready;
+  uint8_t* V = sm + kS * kTile;  // the T tiles T0 .. T7, then the v stage [slice][plane]
+  __shared__ uint64_t v_full, v_empty, acc_full[2], acc_empty[2], e_full[2], y_done, stage_zeroed, t_ready;
   __shared__ uint32_t tmem_slot;
-  __shared__ int e_stage[2], e_acc[2];
-  __shared__ unsigned int red[2][kProdWarps];
+  __shared__ int e_line[2][2][64];          // [item & 1][plane][line]: the lines' exponents
+  __shared__ uint4 line_max[3][16];         // upper words of the lines' largest |v|, three planes in turn
   __shared__ int prod_go, failed, skip;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Planes64<kXY> pg{a.nx, a.ny, a.nz};
-  const int npairs = (a.nplanes + 1) / 2, p_first = blockIdx.x, p_stride = gridDim.x;
+  const Items64<kXY> first{(int)blockIdx.x, (int)gridDim.x, (a.nplanes + 1) / 2};
 
   // a time-out recorded before this launch: leave before any allocation or wait
   if (tid == 0) skip = *(volatile int*)(a.status + 3);
+  if (tid < 48) line_max[tid >> 4][tid & 15] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
   if (skip) return;
   if (tid == 0) {
     tc::mbar_init(&v_full, kProdThreads);
     tc::mbar_init(&v_empty, 1);
-    tc::mbar_init(&acc_full, 1);
-    tc::mbar_init(&acc_empty, kEpiThreads);
-    tc::mbar_init(&e_full, 1);
+    for (int h = 0; h < 2; ++h) {
+      tc::mbar_init(&acc_full[h], 1);
+      tc::mbar_init(&e_full[h], 1);
+      tc::mbar_init(&acc_empty[h], kEpiThreads / 2);
+    }
+    tc::mbar_init(&y_done, kEpiThreads);
     tc::mbar_init(&stage_zeroed, kEpiThreads);
     tc::mbar_init(&t_ready, kEpiThreads);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kMmaWarp) tc::tmem_alloc(&tmem_slot, 512);
+  if (warp == kMmaWarp) tc::tmem_alloc(&tmem_slot, 2 * kAccCols);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -173,96 +242,111 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
   pdl_launch_dependents();
 
   if (warp < kEpiWarps) {
-    // ---- epilogue: TMEM lane quadrant warp % 4 = (plane p, 32-column block of
-    // x), columns [32 half, 32 half + 32) ----
+    // ---- epilogue: TMEM lane quadrant warp % 4 = (plane p, 32-line block),
+    // half of the columns; a lane is a line: the plane's column x of a
+    // contraction over its rows, its row of a contraction along x ----
     const int quad = warp & 3, half = warp >> 2;
-    const int p = quad >> 1, x = ((quad & 1) << 5) + lane;
-    const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-    const long long cstride = pg.row_stride();
-    const int c_begin = half * 32, c_end = min(half * 32 + 32, pg.rows());
+    const int p = quad >> 1, line = ((quad & 1) << 5) + lane;
+    const uint32_t tbase = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)half * kAccCols;
+    const int rstride = pg.row_stride(), rows = pg.rows();
     // the v stage zeroed (the producers write only the groups that hold data),
     // then the T tiles
-    for (int e = tid; e < (int)(2 * kPlane / 16); e += kEpiThreads) reinterpret_cast<uint4*>(V)[e] = make_uint4(0u, 0u, 0u, 0u);
+    for (int e = tid; e < (int)(kS * kPair / 16); e += kEpiThreads) reinterpret_cast<uint4*>(V)[e] = make_uint4(0u, 0u, 0u, 0u);
     tc::fence_smem_to_async();
     tc::mbar_arrive(&stage_zeroed);
     for (int e = tid; e < a.timage16; e += kEpiThreads) reinterpret_cast<uint4*>(sm)[e] = a.timage[e];
     tc::fence_smem_to_async();
     tc::mbar_arrive(&t_ready);
     pdl_wait();  // the output (and, for z, the values added to) belong to earlier kernels
-    for (int it = 0, pair = p_first; pair < npairs; pair += p_stride, ++it) {
+    int it = 0;
+    for (Items64<kXY> w = first; w.more(); w.next(), ++it) {
       const uint32_t par = (uint32_t)it & 1u;
-      const int plane = 2 * pair + p;
-      const bool valid = plane < a.nplanes && x < a.nx;
-      const long long ob = valid ? pg.base(plane) + x : 0;
-      double nxt[4];  // z: the values added to, loaded while the products run
+      const int plane = 2 * w.pair + p;
+      const int nlines = w.along_x ? rows : a.nx, n = w.along_x ? a.nx : rows;
+      const bool valid = plane < a.nplanes && line < nlines;
+      const long long base = valid ? pg.base(plane) + (w.along_x ? line * rstride : line) : 0;
+      const int cstride = w.along_x ? 1 : rstride, mid = half_rows(n);
+      const int c_begin = half * mid, c_end = half ? n : min(mid, n);
+      double* out = a.out + base;
+      const bool add = !kXY || w.along_x;
+      double nxt[4];  // the values added to, loaded while the products run
       auto load4 = [&](int c0) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) nxt[u] = (valid && c0 + u < c_end) ? a.out[ob + (c0 + u) * cstride] : 0.0;
+        for (int u = 0; u < 4; ++u) nxt[u] = (valid && c0 + u < c_end) ? out[(c0 + u) * cstride] : 0.0;
       };
-      if (!kXY) load4(c_begin);
-      int ok = 1;
-      if (lane == 0) ok = tc::mbar_wait(&acc_full, par) && tc::mbar_wait(&e_full, par);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) {
+      // lane 0 waits (bounded) and the warp leaves together on a time-out; every
+      // lane's own wait then returns at once and orders its accesses
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        int ok = lane == 0 ? tc::mbar_wait(bar, parity) : 1;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        return ok && tc::mbar_wait(bar, parity);
+      };
+      // along x other threads of this CTA wrote the sums along y that are added to
+      bool ok = !kXY || !w.along_x || wait(&y_done, (uint32_t)(it >> 1) & 1u);
+      if (ok && add) load4(c_begin);
+      ok = ok && wait(&acc_full[half], par) && wait(&e_full[half], par);
+      if (__any_sync(0xffffffffu, !ok)) {
         failed = 1;
         break;
       }
-      tc::mbar_wait(&acc_full, par);
-      tc::mbar_wait(&e_full, par);
       tc::fence_after_sync();
-      const int e = e_acc[p];
-      const int s = e + a.e_t - 16 - 41;
-      const uint32_t tbase = tmem + lane_base;
+      const int e = e_line[par][p][line];
+      const LineScale q(e == kNonFinite ? 0 : e + a.e_t - 43);
 #pragma unroll 1
       for (int c0 = c_begin; c0 < c_end; c0 += 4) {
         double r[4], cur[4];
-        if (!kXY) {
+        if (add) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
           if (c0 + 4 < c_end) load4(c0 + 4);
         }
-        combine4(tbase + (uint32_t)c0, s, r);
-        if (e == kNonFinite)
+        combine4(tbase + (uint32_t)(c0 - c_begin), q, r);
+        if (e == kNonFinite && valid)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) r[u] = __longlong_as_double(0x7ff8000000000000ll);
+          for (int u = 0; u < 4; ++u)
+            if (c0 + u < c_end) r[u] = plain_sum(a.t + (c0 + u) * n, a.v + base, cstride, n);
         if (valid)
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            if (c0 + u < c_end) a.out[ob + (c0 + u) * cstride] = kXY ? r[u] : r[u] + cur[u];
+            if (c0 + u < c_end) out[(c0 + u) * cstride] = add ? r[u] + cur[u] : r[u];
+        __syncwarp();
       }
       tc::fence_before_sync();
-      tc::mbar_arrive(&acc_empty);
+      tc::mbar_arrive(&acc_empty[half]);
+      if (kXY && !w.along_x) tc::mbar_arrive(&y_done);
     }
   } else if (warp < kMmaWarp) {
-    // ---- producers: item i = (row, 4-column group) of a plane ----
-    const int ptid = tid - kEpiThreads, pw = ptid >> 5;
-    const int nrows = pg.rows(), nx = a.nx, ncg = (nx + 3) >> 2, nitems = nrows * ncg;
-    const long long rstride = pg.row_stride();
-    int goff[kMaxItems], cnt[kMaxItems];
-    uint32_t soff[kMaxItems];
+    // ---- producers: piece i = (row, 4-column group) of a plane ----
+    const int ptid = tid - kEpiThreads;
+    const int nx = a.nx, rstride = pg.row_stride(), ncg = (nx + 3) >> 2, npieces = pg.rows() * ncg;
+    int row[kMaxItems], col[kMaxItems], cnt[kMaxItems];  // cnt 0: no such piece
 #pragma unroll
     for (int t = 0; t < kMaxItems; ++t) {
       const int i = ptid + t * kProdThreads;
-      const int j = i / ncg, c = (i - j * ncg) * 4;
-      const bool iv = i < nitems;
-      goff[t] = iv ? (int)(j * rstride) + c : 0;
-      soff[t] = iv ? quad_offset64(j, c) : 0u;
-      cnt[t] = iv ? min(4, nx - c) : 0;
+      const bool iv = i < npieces;
+      row[t] = iv ? i / ncg : 0;
+      col[t] = iv ? (i - row[t] * ncg) * 4 : 0;
+      cnt[t] = iv ? min(4, nx - col[t]) : 0;
     }
     double x[kMaxItems][4];
-    auto load_item = [&](int t, const double* src) {  // src null: past the last plane
+    auto load_piece = [&](int t, const double* src) {  // src null: past the last plane
+      const double* q = src + (row[t] * rstride + col[t]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) x[t][u] = (src && u < cnt[t]) ? __ldg(src + goff[t] + u) : 0.0;
+      for (int u = 0; u < 4; ++u) x[t][u] = (src && u < cnt[t]) ? __ldg(q + u) : 0.0;
     };
-    auto plane_ptr = [&](int plane) { return plane < a.nplanes ? a.v + pg.base(plane) : nullptr; };
+    auto plane_ptr = [&](const Items64<kXY>& w, int pl) {
+      const int plane = 2 * w.pair + pl;
+      return w.more() && plane < a.nplanes ? a.v + pg.base(plane) : nullptr;
+    };
     pdl_wait();  // v is written by an earlier kernel
+    Items64<kXY> w = first;
     {
-      const double* src = plane_ptr(2 * p_first);
+      const double* src = plane_ptr(w, 0);
 #pragma unroll
-      for (int t = 0; t < kMaxItems; ++t) load_item(t, src);
+      for (int t = 0; t < kMaxItems; ++t) load_piece(t, src);
     }
     int slot = 0;
-    for (int it = 0, pair = p_first; pair < npairs; pair += p_stride, ++it) {
+    for (int it = 0; w.more(); ++it) {
       const uint32_t par = (uint32_t)it & 1u;
       if (ptid == 0)
         prod_go = ((it > 0 || tc::mbar_wait(&stage_zeroed, 0u)) && tc::mbar_wait(&v_empty, par ^ 1u)) ? 1 : 0;
@@ -271,42 +355,64 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
         if (ptid == 0) failed = 1;
         break;
       }
+      const bool along_x = w.along_x;
 #pragma unroll 1
       for (int pl = 0; pl < 2; ++pl) {
-        unsigned int mx = 0u;
+        // the largest |v| of every line (by the upper words), over the plane's pieces
+        unsigned int* mx = reinterpret_cast<unsigned int*>(line_max[slot]);
 #pragma unroll
         for (int t = 0; t < kMaxItems; ++t)
+          if (cnt[t] > 0) {
+            unsigned int hi[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mx = max(mx, (unsigned int)__double2hiint(x[t][u]) & 0x7fffffffu);
-        mx = __reduce_max_sync(0xffffffffu, mx);
-        if (lane == 0) red[slot][pw] = mx;
+            for (int u = 0; u < 4; ++u) hi[u] = (unsigned int)__double2hiint(x[t][u]) & 0x7fffffffu;
+            if (kXY && along_x) {
+              atomicMax(mx + row[t], max(max(hi[0], hi[1]), max(hi[2], hi[3])));
+            } else {
+#pragma unroll
+              for (int u = 0; u < 4; ++u) atomicMax(mx + col[t] + u, hi[u]);
+            }
+          }
         tc::named_sync(1, kProdThreads);
-#pragma unroll
-        for (int w = 0; w < kProdWarps; ++w) mx = max(mx, red[slot][w]);
-        slot ^= 1;
-        // |v| < 2^e over the plane (0 for a plane of zeros and subnormals)
-        const int e = mx >= 0x7ff00000u ? kNonFinite : (mx >> 20) ? (int)(mx >> 20) - 1022 : 0;
-        if (ptid == 0) e_stage[pl] = e;
-        uint8_t* vp = V + pl * kPlane;
-        // the next plane's values are loaded item by item as this one's are sliced
-        const double* next = plane_ptr(pl == 0 ? 2 * pair + 1 : 2 * (pair + p_stride));
+        // the slot of the plane after next: last read before this barrier, next written after the next one
+        const int clear = slot == 0 ? 2 : slot - 1;
+        if (ptid < 64) {
+          reinterpret_cast<unsigned int*>(line_max[clear])[ptid] = 0u;
+          e_line[par][pl][ptid] = line_exponent(mx[ptid]);
+        }
+        slot = slot == 2 ? 0 : slot + 1;
+        uint8_t* vp = V + pl * kTile;
+        // the next plane's values are loaded piece by piece as this one's are sliced
+        if (pl == 1) w.next();
+        const double* next = plane_ptr(w, pl ^ 1);
 #pragma unroll
         for (int t = 0; t < kMaxItems; ++t) {
           if (cnt[t] > 0) {
-            unsigned long long f[4];
+            uint4 h;
+            if (kXY && along_x) {
+              h.x = h.y = h.z = h.w = mx[row[t]];
+            } else {
+              h = reinterpret_cast<const uint4*>(mx)[col[t] >> 2];
+            }
+            const unsigned int hs[4] = {h.x, h.y, h.z, h.w};
+            Digits f[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) f[u] = fixed_point(x[t][u], e);
-            uint8_t* dst = vp + soff[t];
-            // slice k (most significant first) is digit 6 - k
-            *reinterpret_cast<uint2*>(dst) = make_uint2(slice2<6>(f[0], f[1]), slice2<6>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + kTile) = make_uint2(slice2<5>(f[0], f[1]), slice2<5>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + 2 * kTile) = make_uint2(slice2<4>(f[0], f[1]), slice2<4>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + 3 * kTile) = make_uint2(slice2<3>(f[0], f[1]), slice2<3>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + 4 * kTile) = make_uint2(slice2<2>(f[0], f[1]), slice2<2>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + 5 * kTile) = make_uint2(slice2<1>(f[0], f[1]), slice2<1>(f[2], f[3]));
-            *reinterpret_cast<uint2*>(dst + 6 * kTile) = make_uint2(slice2<0>(f[0], f[1]), slice2<0>(f[2], f[3]));
+            for (int u = 0; u < 4; ++u) f[u] = digits_of(x[t][u], max((int)(hs[u] >> 20), 1));
+            uint8_t* dst = vp + quad_offset64(row[t], col[t]);
+            // slice k, the most significant first
+            auto put = [&](int k, uint32_t lo, uint32_t hi) {
+              *reinterpret_cast<uint2*>(dst + k * kPair) = make_uint2(lo, hi);
+            };
+            put(0, slice2<3>(f[0].hi, f[1].hi), slice2<3>(f[2].hi, f[3].hi));
+            put(1, slice2<2>(f[0].hi, f[1].hi), slice2<2>(f[2].hi, f[3].hi));
+            put(2, slice2<1>(f[0].hi, f[1].hi), slice2<1>(f[2].hi, f[3].hi));
+            put(3, slice2<0>(f[0].hi, f[1].hi), slice2<0>(f[2].hi, f[3].hi));
+            put(4, slice2<3>(f[0].lo, f[1].lo), slice2<3>(f[2].lo, f[3].lo));
+            put(5, slice2<2>(f[0].lo, f[1].lo), slice2<2>(f[2].lo, f[3].lo));
+            put(6, slice2<1>(f[0].lo, f[1].lo), slice2<1>(f[2].lo, f[3].lo));
+            put(7, slice2<0>(f[0].lo, f[1].lo), slice2<0>(f[2].lo, f[3].lo));
           }
-          load_item(t, next);
+          load_piece(t, next);
         }
       }
       tc::fence_smem_to_async();
@@ -315,59 +421,43 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
   } else if (lane == 0) {
     // ---- MMA issue ----
     const uint32_t tb = tc::smem_u32(sm), vb = tc::smem_u32(V);
-    const uint32_t t0 = tb + (kXY ? kTile : 0u);
-    // 16-row steps of the contractions that hold data (the rest is zero padding)
+    // A = a slice of the pair: M = (p, x) over the rows (MN-major, the planes kTile
+    // apart) or M = (p, row) along x (K-major, 128 rows); B = T slices stacked along N
+    const uint64_t a_rows = tc::sw128_mn_desc(vb, kTile, 1024u), a_x = tc::sw128_desc(vb), b0 = tc::sw128_desc(tb);
+    // 16-wide steps of the contractions that hold data (the rest is zero padding)
     const int ks_rows = (pg.rows() + 15) / 16, ks_x = (a.nx + 15) / 16;
     if (!tc::mbar_wait(&t_ready, 0u)) failed = 1;
-    for (int it = 0, pair = p_first; pair < npairs && !failed; pair += p_stride, ++it) {
+    int it = 0;
+    for (Items64<kXY> w = first; w.more() && !failed; w.next(), ++it) {
       const uint32_t par = (uint32_t)it & 1u;
-      if (!tc::mbar_wait(&v_full, par) || !tc::mbar_wait(&acc_empty, par ^ 1u)) {
+      if (!tc::mbar_wait(&v_full, par)) {
         failed = 1;
         break;
       }
-      tc::fence_after_sync();
-      e_acc[0] = e_stage[0];
-      e_acc[1] = e_stage[1];
-      tc::mbar_arrive(&e_full);
-      // Class c accumulates in columns [64 c, 64 c + 64).  An MMA whose B stacks
-      // slices l0 .. l0 + n - 1 along N (at most four: N <= 256) and whose D
-      // starts at column 64 (k + l0) puts product (k, l) into class k + l.
-      // Contraction over the rows of each plane: A = v slice k (M = (p, x),
-      // MN-major, the planes kPlane apart), B = T slices.  Slice 0 of v sets
-      // every class.
+      // Class c of a half accumulates in its columns [32 c, 32 c + 32).  The MMA of
+      // v's slice k stacks T's slices 0 .. 7 - k along N and starts at class k, so
+      // that product (k, l) goes into class k + l; slice 0 sets every class.
+      const bool x = kXY && w.along_x;
+      const uint64_t a0 = x ? a_x : a_rows;
+      const uint32_t astep = x ? 32u / 16u : 2048u / 16u, major = x ? 0u : tc::kIdescAMajorMN;
+      const int ks = x ? ks_x : ks_rows;
 #pragma unroll 1
-      for (int k = 0; k < kS; ++k)
-#pragma unroll 1
-        for (int l0 = 0; l0 < kS - k; l0 += 4) {
-          const uint32_t idesc = tc::idesc_f16(128, 64 * min(4, kS - k - l0)) | tc::kIdescAMajorMN;
-          for (int s = 0; s < ks_rows; ++s)
-            tc::mma_f16(tmem + 64u * (uint32_t)(k + l0),
-                        tc::sw128_mn_desc(vb + (uint32_t)k * kTile + (uint32_t)s * 2048u, kPlane, 1024u),
-                        tc::sw128_desc(t0 + (uint32_t)l0 * kTile + (uint32_t)s * 32u), idesc,
-                        (k == 0 && s == 0) ? 0u : 1u);
+      for (uint32_t half = 0; half < 2; ++half) {
+        if (!tc::mbar_wait(&acc_empty[half], par ^ 1u)) {
+          failed = 1;
+          break;
         }
-      if (kXY) {
-        // contraction along x: A = diag(T_l, T_l) over K = (p', q), read MN-major
-        // (T is symmetric), B = v slices of plane p' stacked along N
-        const uint32_t zlo = tb, zhi = tb + (uint32_t)(kS + 1) * kTile;
-#pragma unroll 1
-        for (int l = 0; l < kS; ++l) {
-          const uint32_t tl = t0 + (uint32_t)l * kTile;
-#pragma unroll 1
-          for (int k0 = 0; k0 < kS - l; k0 += 4) {
-            const uint32_t idesc = tc::idesc_f16(128, 64 * min(4, kS - l - k0)) | tc::kIdescAMajorMN;
-            for (uint32_t pp = 0; pp < 2; ++pp)
-              for (uint32_t q = 0; q < (uint32_t)ks_x; ++q) {
-                const uint64_t adesc = pp ? tc::sw128_mn_desc(zlo + q * 2048u, tl - zlo, 1024u)
-                                          : tc::sw128_mn_desc(tl + q * 2048u, zhi - tl, 1024u);
-                tc::mma_f16(tmem + 64u * (uint32_t)(l + k0), adesc,
-                            tc::sw128_desc(vb + pp * kPlane + (uint32_t)k0 * kTile + q * 32u), idesc, 1u);
-              }
-          }
-        }
+        tc::fence_after_sync();
+        tc::mbar_arrive(&e_full[half]);
+        const uint64_t bd = b0 + half * (kS * kHalfTile / 16u);
+#pragma unroll
+        for (int k = 0; k < kS; ++k)
+          for (int i = 0; i < ks; ++i)
+            tc::mma_f16(tmem + half * kAccCols + 32u * k, a0 + (uint32_t)k * (kPair / 16u) + (uint32_t)i * astep,
+                        bd + (uint32_t)i * 2u, tc::idesc_f16(128, 32 * (kS - k)) | major, (k == 0 && i == 0) ? 0u : 1u);
+        if (half) tc::mma_commit(&v_empty);
+        tc::mma_commit(&acc_full[half]);
       }
-      tc::mma_commit(&v_empty);
-      tc::mma_commit(&acc_full);
     }
   }
   tc::fence_before_sync();
@@ -375,19 +465,18 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
   if (failed && tid == 0) a.status[3] = 1;
   if (warp == kMmaWarp) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem, 512);
+    tc::tmem_dealloc(tmem, 2 * kAccCols);
   }
 }
 
-// x and y contractions: out(y, x) = Tx v + Ty v
+// x and y contractions: out(y, x) = Ty v, then + Tx v
 __global__ void __launch_bounds__(kThreads64, 1) k_kin_xy_tc64(Kin64 a) { kin64_body<true>(a); }
 // z contraction added: out(z, x) += Tz v
 __global__ void __launch_bounds__(kThreads64, 1) k_kin_z_tc64(Kin64 a) { kin64_body<false>(a); }
 
-constexpr size_t kSmemXY = 1024 + (kS + 2) * kTile + 2 * kPlane;
-constexpr size_t kSmemZ = 1024 + kS * kTile + 2 * kPlane;
-static_assert(kSmemXY + 512 <= 227 * 1024, "x/y T tiles and the stage must fit in one CTA's shared memory");
-static_assert(kAccCols <= 512, "the accumulator must fit in tensor memory");
+constexpr size_t kSmem64 = 1024 + kS * kTile + kS * kPair;
+static_assert(kSmem64 + 3072 <= 227 * 1024, "the T tiles and the stage must fit in one CTA's shared memory");
+static_assert(2 * kAccCols <= 512, "the accumulator must fit in tensor memory");
 
 uint16_t half_bits(int x) {
   const __half h = __float2half_rn((float)x);
@@ -398,35 +487,46 @@ uint16_t half_bits(int x) {
 
 }  // namespace
 
-// The seven 9-bit slices of a symmetric T (62 bits below 2^e_t > max|T|, rounded
-// to nearest, digits in [-256, 256]) as the kernels' shared-memory T region.
-void kinetic_smem_image64(const std::vector<double>& T, int n, bool with_zero_tiles, std::vector<uint16_t>* image,
-                          int* e_t) {
+// The eight 9-bit slices of a symmetric T, [half][slice] (71 bits below 2^e_t > max|T|, digits in
+// [-256, 256]) as the kernels' shared-memory T region.  False when a class sum
+// that has to be exact (0-6) could come near 2^24 for some v: 256 times the sum
+// of |digit| over a row and the slices up to the class's above 15 2^20.  The
+// sinc-DVR matrices up to 64 points reach 0.8 of 2^24, and 2^22 in class 1.
+bool kinetic_smem_image64(const std::vector<double>& T, int n, std::vector<uint16_t>* image, int* e_t) {
   double m = 0.0;
   for (double x : T) m = std::max(m, std::fabs(x));
   int e = 0;
   if (m > 0.0) std::frexp(m, &e);
   *e_t = e;
-  const int first = with_zero_tiles ? 1 : 0;
-  image->assign((size_t)(kS + 2 * first) * kTile / 2, half_bits(0));
-  for (int i = 0; i < n; ++i)
+  image->assign((size_t)kS * kTile / 2, half_bits(0));
+  const __int128 bias = ((__int128)kBias36 << 36) + kBias36;
+  long long most = 0, first = 0;
+  for (int i = 0; i < n; ++i) {
+    long long row = 0, two = 0;
     for (int q = 0; q < n; ++q) {
-      // |T| 2^(62 - e) < 2^62 is exact to the last FP64 bit where |T| >= 2^(e - 10)
-      const unsigned long long f = kBias + (unsigned long long)std::llrint(std::ldexp(T[(size_t)i * n + q], 62 - e));
+      const __int128 f = bias + (__int128)std::nearbyint(std::ldexp(T[(size_t)i * n + q], 71 - e));
       for (int l = 0; l < kS; ++l) {
         const int digit = kS - 1 - l;
-        const int b = (int)((f >> (9 * digit)) & (digit == kS - 1 ? 0x3ffull : 0x1ffull)) - 256;
-        const size_t byte = (size_t)(first + l) * kTile + (size_t)i * 128 + (size_t)(((q >> 3) ^ (i & 7)) << 4) +
-                            (size_t)(q & 7) * 2;
+        const int b = (int)((f >> (9 * digit)) & (digit == kS - 1 ? 0x3ff : 0x1ff)) - 256;
+        if (l < kS - 1) row += std::abs(b);
+        if (l < 2) two += std::abs(b);
+        const int half = i >= half_rows(n), r = i - half * half_rows(n);
+        const size_t byte = (size_t)(half * kS + l) * kHalfTile + (size_t)r * 128 +
+                            (size_t)(((q >> 3) ^ (r & 7)) << 4) + (size_t)(q & 7) * 2;
         (*image)[byte / 2] = half_bits(b);
       }
     }
+    most = std::max(most, row);
+    first = std::max(first, two);
+  }
+  return 256 * most <= 15ll << 20 && 256 * first < 4000000;
 }
 
 int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s) {
   const Tables& t = h->t;
   DeviceState& d = h->d;
   Kin64 a{};
+  a.t = xy ? d.tx : d.tz;
   a.v = v;
   a.out = d.ukin;
   a.nx = t.nx;
@@ -434,7 +534,7 @@ int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s) {
   a.nz = t.nz;
   a.status = d.status;
   a.timage = reinterpret_cast<const uint4*>(xy ? d.kxy_slices64 : d.kz_slices64);
-  a.timage16 = (int)((xy ? kS + 2 : kS) * kTile / 16);
+  a.timage16 = (int)(kS * kTile / 16);
   a.e_t = xy ? d.e_txy64 : d.e_tz64;
   a.nplanes = (xy ? t.nz : t.ny) * t.nn;
   int dev = 0, sms = 0;
@@ -442,11 +542,11 @@ int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const dim3 grid(std::min((a.nplanes + 1) / 2, std::max(1, sms)));
   if (xy) {
-    cudaFuncSetAttribute(k_kin_xy_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemXY);
-    BSL_CUDA(launch_pdl(k_kin_xy_tc64, grid, dim3(kThreads64), kSmemXY, s, a));
+    cudaFuncSetAttribute(k_kin_xy_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem64);
+    BSL_CUDA(launch_pdl(k_kin_xy_tc64, grid, dim3(kThreads64), kSmem64, s, a));
   } else {
-    cudaFuncSetAttribute(k_kin_z_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemZ);
-    BSL_CUDA(launch_pdl(k_kin_z_tc64, grid, dim3(kThreads64), kSmemZ, s, a));
+    cudaFuncSetAttribute(k_kin_z_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem64);
+    BSL_CUDA(launch_pdl(k_kin_z_tc64, grid, dim3(kThreads64), kSmem64, s, a));
   }
   return BSL_OK;
 }
