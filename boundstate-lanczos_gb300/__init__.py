@@ -334,7 +334,7 @@ class Hamiltonian:
         _check(lib().bsl_set_precision(self._h, PREC[precision]))
 
     def set_kinetic_engine(self, engine):
-        """Kinetic engine of the mixed precision: "simt" or "tensor"."""
+        """Kinetic engine: "simt" (in FP64 the plain sums) or "tensor"."""
         _check(lib().bsl_set_kinetic_engine(self._h, KINETIC[engine]))
 
     def set_kinetic_slices(self, slices):

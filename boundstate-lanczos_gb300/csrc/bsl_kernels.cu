@@ -776,7 +776,7 @@ int launch_kinetic(bsl_handle* h, const double* v, const float2* vpair, cudaStre
 // us at 21^3 (1.2e7), 62 against 52 us at 24^3 (2.1e7), 993 against 127 us at 54^3.
 bool kin_f64_tensor(const bsl_handle* h) {
   const Tables& t = h->t;
-  return h->d.kxy_slices64 && (double)t.npts * t.nn * (t.nx + t.ny + t.nz) >= 1.6e7;
+  return h->kinetic_engine == BSL_KIN_TENSOR && h->d.kxy_slices64 && (double)t.npts * t.nn * (t.nx + t.ny + t.nz) >= 1.6e7;
 }
 
 // ---------------------------------------------------------------------------

@@ -62,14 +62,20 @@ extern "C" {
                                        origin and one on the H2 centre of mass */
 
 /* arithmetic of the Hv application */
-#define BSL_PREC_FP64 0  /* every step in FP64 */
+#define BSL_PREC_FP64 0  /* every step in FP64 or, the kinetic contractions of larger
+                            problems with BSL_KIN_TENSOR, in integers: every element
+                            of T v within one FP64 rounding of the sum of its own
+                            |T v| terms in each direction, where an FP64 sum of n
+                            terms may be off by n of them */
 #define BSL_PREC_MIXED 1 /* FP32 potential values, an FP32 / tensor-core kinetic
                             exact to ~2^-36 (or FP32 head and tail coefficients
                             on the CUDA cores), double-float rotor diagonal and
                             double-float (~48-bit) Lanczos recurrence; grids of
                             at most 64 points per axis (the kinetic engines) */
 
-/* engine of the FP32 kinetic contractions in BSL_PREC_MIXED */
+/* engine of the kinetic contractions.  In BSL_PREC_FP64, BSL_KIN_SIMT forms plain
+   FP64 sums at every size; BSL_KIN_TENSOR cuts each contracted line of v into
+   eight integer slices where that is faster.  In BSL_PREC_MIXED: */
 #define BSL_KIN_SIMT 0   /* FP32 head/tail coefficients on the CUDA cores; grids of
                             at most 64 points per axis: one thread owns a 4 x 4
                             tile of a plane's output and a CTA of at most 256
@@ -172,13 +178,13 @@ int bsl_packed_nn(const bsl_handle* h);
 /* Switch the arithmetic of later Hv applications (BSL_PREC_*). */
 int bsl_set_precision(bsl_handle* h, int precision);
 
-/* Select the kinetic engine of BSL_PREC_MIXED (BSL_KIN_*).  bsl_hv_prep selects
+/* Select the kinetic engine (BSL_KIN_*).  bsl_hv_prep selects
    BSL_KIN_TENSOR where the grid allows it (at most 64 points per axis, equal x
    and y axes), else BSL_KIN_SIMT; BSL_ERR_UNSUPPORTED when the grid does not
-   allow BSL_KIN_TENSOR.  The tensor engine slices the double-float Lanczos
-   vector exactly into FP16 fixed-point parts and accumulates exactly: its H v
-   deviates from the FP64 path by ~3e-9 relative, the CUDA-core engine's by
-   ~2e-7. */
+   allow BSL_KIN_TENSOR.  In BSL_PREC_MIXED the tensor engine slices the
+   double-float Lanczos vector exactly into FP16 fixed-point parts and
+   accumulates exactly: its H v deviates from the FP64 path by ~3e-9 relative,
+   the CUDA-core engine's by ~2e-7. */
 int bsl_set_kinetic_engine(bsl_handle* h, int engine);
 int bsl_kinetic_engine(const bsl_handle* h);
 

@@ -96,3 +96,30 @@ def test_an_infinity_reaches_its_own_lines_only(bsl):
         assert np.all(u == 0.0)
     finally:
         h.close()
+
+
+def test_the_cuda_core_engine_selects_the_plain_sums(bsl):
+    """In FP64 as well: the same H v from one kernel and the other, and the tensor
+    cores' no further off on average, element by element."""
+    n = (57, 57, 57)
+    h = bare(bsl, n)
+    try:
+        t = [sinc_dvr_t(k).astype(np.longdouble) for k in n]
+        v = vectors(n, np.random.default_rng(1))["bound state"]
+        i = np.random.default_rng(2).integers(0, 57, (4000, 3))
+        x, y, z = i.T
+        w = v.astype(np.longdouble)
+        parts = [t[0][x] * w[z, y, :], t[1][y] * w[z, :, x], t[2][z] * w[:, y, x].T]
+        exact, terms = sum(p.sum(1) for p in parts), sum(np.abs(p).sum(1) for p in parts)
+        rms = []
+        for engine, launches in (("simt", 3), ("tensor", 4)):
+            h.set_kinetic_engine(engine)
+            assert bsl.lib().bsl_launches_per_iteration(C.c_void_p(h.handle.value)) == launches
+            u = np.zeros(v.size)
+            h.hv(v.ravel(), u)
+            off = np.abs(u.reshape(v.shape)[z, y, x] - exact) / terms
+            assert np.max(off) <= sum(n) * 2.0 ** -53
+            rms.append(float(np.sqrt(np.mean(off ** 2))))
+        assert rms[1] <= rms[0], rms
+    finally:
+        h.close()
