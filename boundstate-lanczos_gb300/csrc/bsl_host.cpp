@@ -784,7 +784,7 @@ int bsl_hv_apply(bsl_handle* h, const double* vec, double* uec) {
   BSL_CUDA(cudaMemcpyAsync(st, d.status, sizeof(st), cudaMemcpyDeviceToHost, s));
   BSL_CUDA(cudaStreamSynchronize(s));
   if (st[2] || st[3]) {
-    cudaMemset(d.status, 0, sizeof(st));  // reported: later calls start clean
+    if ((rc = clear_status(h))) return rc;  // reported: later calls start clean
     return fail(BSL_ERR_CUDA, st[2] ? "potential-block stream: a bulk copy did not complete within its time limit"
                                     : "tensor-core kinetic: an MMA did not complete within its time limit");
   }

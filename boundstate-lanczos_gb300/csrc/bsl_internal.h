@@ -340,6 +340,7 @@ int dev_gaunt_coeffs(bsl_handle* h, double* residual, double* vmax);
 
 // host-layout staging buffers, the second copy stream and its events (bsl_lanczos.cpp)
 int ensure_staging(bsl_handle* h);
+int clear_status(bsl_handle* h);
 // the cached iteration graph (bsl_lanczos.cpp)
 void release_iteration_graph(DeviceState& d);
 

@@ -44,6 +44,15 @@ int ensure_staging(bsl_handle* h) {
   return BSL_OK;
 }
 
+// The status words cleared, and seen cleared by every later call: on the
+// library's stream (which does not wait for the legacy stream) and waited for,
+// since bsl_hv_apply_device may be given another one.
+int clear_status(bsl_handle* h) {
+  BSL_CUDA(cudaMemsetAsync(h->d.status, 0, 4 * sizeof(int), h->d.stream));
+  BSL_CUDA(cudaStreamSynchronize(h->d.stream));
+  return BSL_OK;
+}
+
 namespace {
 
 // The history buffer grows in steps of kHistStep iterations, so runs of
@@ -144,9 +153,11 @@ int init_state(bsl_handle* h, int start, unsigned long long seed) {
 
 int check_status(bsl_handle* h) {
   int st[4] = {0, 0, 0, 0};
-  BSL_CUDA(cudaMemcpy(st, h->d.status, 4 * sizeof(int), cudaMemcpyDeviceToHost));
+  BSL_CUDA(cudaMemcpyAsync(st, h->d.status, sizeof(st), cudaMemcpyDeviceToHost, h->d.stream));
+  BSL_CUDA(cudaStreamSynchronize(h->d.stream));
   // a time-out is reported once: kernels launched outside a run (H v) read the words too
-  if (st[2] || st[3]) BSL_CUDA(cudaMemset(h->d.status, 0, 4 * sizeof(int)));
+  if (st[2] || st[3])
+    if (int rc = clear_status(h)) return rc;
   if (st[2]) return fail(BSL_ERR_CUDA, "potential-block stream: a bulk copy did not complete within its time limit");
   if (st[3]) return fail(BSL_ERR_CUDA, "tensor-core kinetic: an MMA did not complete within its time limit");
   if (st[0]) return fail(BSL_ERR_BREAKDOWN, "Lanczos breakdown at iteration " + std::to_string(st[1]) +
