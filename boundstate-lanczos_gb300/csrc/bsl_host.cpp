@@ -753,6 +753,8 @@ int bsl_hv_apply_device(bsl_handle* h, const double* d_v, double* d_u, void* str
   if (!h) return fail(BSL_ERR_STATE, "null handle");
   if (!d_v || !d_u) return fail(BSL_ERR_INPUT, "null argument");
   cudaSetDevice(h->p.device);
+  if (h->d.inject_status)
+    if (int rc = reset_status(h, (cudaStream_t)stream)) return rc;
   return dev_hv(h, d_v, d_u, (cudaStream_t)stream);
 }
 

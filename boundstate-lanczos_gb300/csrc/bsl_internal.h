@@ -341,6 +341,8 @@ int dev_gaunt_coeffs(bsl_handle* h, double* residual, double* vmax);
 // host-layout staging buffers, the second copy stream and its events (bsl_lanczos.cpp)
 int ensure_staging(bsl_handle* h);
 int clear_status(bsl_handle* h);
+// status words cleared at the start of a run or step, then the injected ones set
+int reset_status(bsl_handle* h, cudaStream_t s);
 // the cached iteration graph (bsl_lanczos.cpp)
 void release_iteration_graph(DeviceState& d);
 

@@ -201,6 +201,22 @@ __device__ __forceinline__ double plain_sum(const double* trow, const double* v,
   return acc;
 }
 
+// After a time-out: NaN in the planes of the CTA's items, so that an H v whose
+// caller does not read the status words (bsl_hv_apply_device) cannot be taken
+// for a result.
+template <bool kXY>
+__device__ __forceinline__ void poison(const Kin64& a, Items64<kXY> w) {
+  pdl_wait();
+  const Planes64<kXY> pg{a.nx, a.ny, a.nz};
+  for (; w.more(); w.pair += w.stride)
+    for (int e = threadIdx.x; e < 2 * pg.rows() * a.nx; e += blockDim.x) {
+      const int row = e / a.nx, pl = row >= pg.rows(), plane = 2 * w.pair + pl;
+      if (plane < a.nplanes)
+        a.out[pg.base(plane) + (long long)(row - pl * pg.rows()) * pg.row_stride() + e % a.nx] =
+            __longlong_as_double(0x7ff8000000000000ll);
+    }
+}
+
 template <bool kXY>
 __device__ __forceinline__ void kin64_body(const Kin64& a) {
   extern __shared__ uint8_t smraw[];
@@ -219,7 +235,10 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
   if (tid == 0) skip = *(volatile int*)(a.status + 3);
   if (tid < 48) line_max[tid >> 4][tid & 15] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  if (skip) return;
+  if (skip) {
+    poison<kXY>(a, first);
+    return;
+  }
   if (tid == 0) {
     tc::mbar_init(&v_full, kProdThreads);
     tc::mbar_init(&v_empty, 1);
@@ -467,6 +486,7 @@ __device__ __forceinline__ void kin64_body(const Kin64& a) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, 2 * kAccCols);
   }
+  if (failed) poison<kXY>(a, first);
 }
 
 // x and y contractions: out(y, x) = Ty v, then + Tx v

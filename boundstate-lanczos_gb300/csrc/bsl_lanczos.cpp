@@ -53,6 +53,16 @@ int clear_status(bsl_handle* h) {
   return BSL_OK;
 }
 
+// status words cleared at the start of a run or step, then the injected
+// time-out flags of the test hook (bsl_debug_inject_timeout)
+int reset_status(bsl_handle* h, cudaStream_t s) {
+  DeviceState& d = h->d;
+  BSL_CUDA(cudaMemsetAsync(d.status, 0, 4 * sizeof(int), s));
+  for (int w = 2; w <= 3; ++w)
+    if (d.inject_status & (1 << w)) BSL_CUDA(cudaMemsetAsync(d.status + w, 0x01, 1, s));
+  return BSL_OK;
+}
+
 namespace {
 
 // The history buffer grows in steps of kHistStep iterations, so runs of
@@ -69,16 +79,6 @@ int ensure_hist(bsl_handle* h, int niter) {
   d.hist_cap = (niter + 1 + kHistStep - 1) / kHistStep * kHistStep;
   BSL_CUDA(cudaMalloc(&d.hist, 3 * (size_t)d.hist_cap * sizeof(double)));
   BSL_CUDA(cudaMemset(d.hist, 0, 3 * (size_t)d.hist_cap * sizeof(double)));
-  return BSL_OK;
-}
-
-// status words cleared at the start of a run or step, then the injected
-// time-out flags of the test hook (bsl_debug_inject_timeout)
-int reset_status(bsl_handle* h, cudaStream_t s) {
-  DeviceState& d = h->d;
-  BSL_CUDA(cudaMemsetAsync(d.status, 0, 4 * sizeof(int), s));
-  for (int w = 2; w <= 3; ++w)
-    if (d.inject_status & (1 << w)) BSL_CUDA(cudaMemsetAsync(d.status + w, 0x01, 1, s));
   return BSL_OK;
 }
 

@@ -364,6 +364,13 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       }
     }
   }
+  if (kRole == 0 && A.mode == 0 && (abort_flag || *(volatile int*)(A.status + 3))) {
+    // H v on its own, after a time-out here or in the kinetic: NaN in the CTA's
+    // points, so that a caller who does not read the status words
+    // (bsl_hv_apply_device) cannot take them for a result
+    for (long long p = t0 * kTilePts + tid; p < t1 * kTilePts && p < npts; p += kTilePts)
+      for (int s = 0; s < NN; ++s) A.out[s * npts + p] = __longlong_as_double(0x7ff8000000000000ll);
+  }
   if (abort_flag && tid == 0 && issued > 0) {
     // a copy did not complete in time: record it and give the copies still in
     // flight a bounded chance to land before the CTA's shared memory is released

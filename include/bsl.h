@@ -228,7 +228,10 @@ double bsl_gaunt_residual(const bsl_handle* h);
 int bsl_hv_apply(bsl_handle* h, const double* vec, double* uec);
 
 /* u = H v on device buffers in the packed layout, on `stream` (cudaStream_t,
-   NULL = the legacy default stream). */
+   NULL = the legacy default stream).  Only queues its kernels: where one of their
+   bounded waits ran out, u holds NaN, and so does every later u of the handle
+   until a call that waits (bsl_hv_apply, a run or a step) has returned the error
+   or begun anew. */
 int bsl_hv_apply_device(bsl_handle* h, const double* d_v, double* d_u, void* stream);
 
 /* Lanczos loop 1 on the device (lanczosEigenValuesVectors.cpp:170-242): niter
@@ -425,9 +428,10 @@ int bsl_autotune(bsl_handle** hs, int n, int iters, int* vs_per_sm, int* upd_per
    kinetic records a time-out in a device status word, and the next
    bsl_lanczos_run / bsl_lanczos_step_host returns BSL_ERR_CUDA with the
    stage named.  kernel_mask bit 0 (potential stream) and bit 1 (tensor-core
-   kinetic) make every later run or step start with that stage's time-out
-   already recorded: the kernels then skip their copies, MMAs and waits, the
-   results are meaningless and the call returns the error.  0 clears the
+   kinetic) make every later run, step or bsl_hv_apply_device start with that
+   stage's time-out already recorded: the kernels then skip their copies, MMAs
+   and waits, the results are meaningless and the call returns the error
+   (bsl_hv_apply_device: NaN).  0 clears the
    injection; the handle is usable again at once.  Nothing on the GPU is made
    to wait or fault. */
 int bsl_debug_inject_timeout(bsl_handle* h, int kernel_mask);

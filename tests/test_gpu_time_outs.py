@@ -70,3 +70,28 @@ def test_the_next_call_starts_clean_whatever_the_legacy_stream_holds(bsl, precis
             t.join()
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("precision,mask", [("fp64", 2), ("mixed", 1), ("mixed", 2), ("mixed", 3)])
+def test_device_h_v_is_nan_until_a_call_has_reported(bsl, precision, mask):
+    torch = pytest.importorskip("torch")
+    h = hamiltonian(bsl, 30, precision)
+    try:
+        v = torch.randn(21 * 30 ** 3, dtype=torch.float64, device="cuda")
+        ref, u = torch.empty_like(v), torch.zeros_like(v)
+        s = torch.cuda.current_stream().cuda_stream
+        h.hv_device(v.data_ptr(), ref.data_ptr(), s)
+        h.inject_timeout(mask)
+        h.hv_device(v.data_ptr(), u.data_ptr(), s)
+        h.inject_timeout(0)
+        assert bool(torch.isnan(u).all())
+        u.zero_()
+        h.hv_device(v.data_ptr(), u.data_ptr(), s)  # the time-out stands
+        assert bool(torch.isnan(u).all())
+        w = np.zeros(h.basis_size)
+        with pytest.raises(bsl.BslError):
+            h.hv(np.ones(h.basis_size), w)
+        h.hv_device(v.data_ptr(), u.data_ptr(), s)
+        assert torch.equal(u, ref) and bool(torch.isfinite(ref).all())
+    finally:
+        h.close()
