@@ -437,7 +437,7 @@ int hv_prep(const bsl_hv_params* params, const Cage* cage, bsl_handle** out) {
     kinetic_tc_image(t, &sl, &d.kin_tz_tile, &d.e_txy, &d.e_tz);
     d.kin_image16 = (int)(sl.size() * sizeof(uint16_t) / 16);
     if ((rc = upload(&d.kin_slices, sl, "T"))) return bail(rc);
-    if (kin_tc_one_launch(h) && (rc = dalloc(&d.ukin_z, (size_t)t.npts * t.nn, "kinetic work"))) return bail(rc);
+    if (kin_tc_small(t) && (rc = dalloc(&d.ukin_z, (size_t)t.npts * t.nn, "kinetic work"))) return bail(rc);
     std::vector<float> sf;
     kinetic_slices_f32(t.tx, t.nx, &sf);
     if ((rc = upload(&d.tx_slices32, sf, "Tx"))) return bail(rc);

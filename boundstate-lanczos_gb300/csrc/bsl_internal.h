@@ -247,6 +247,7 @@ bool kin_f64_tensor(const bsl_handle* h);
 void kinetic_tc_image(const Tables& t, std::vector<uint16_t>* image, int* tz_tile, int* e_txy, int* e_tz);
 // whether launch_kin_xy_tc forms all three contractions (z in d.ukin_z) and launch_kin_z_tc nothing
 bool kin_tc_one_launch(const bsl_handle* h);
+bool kin_tc_small(const Tables& t);  // whether it is worth its buffer
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 int launch_kin_z_tc(bsl_handle* h, const float2* v, cudaStream_t s);
 // grouped tensor-core kinetic over several problems: per-problem argument
@@ -263,9 +264,8 @@ int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nct
 // FP32 blocks in the tile-major layout of bsl_vstream.cu (vstream_tile_points() points per tile)
 struct StreamArgs {
   const float* vb;      // tile-major FP32 blocks
-  const float* v32;     // FP32 copy of v (mode 0 and 1 of the CUDA-core kinetic)
-  const float2* vpair;  // mode 0 of the tensor-core kinetic: v as pairs, whose heads take its place
-  const double* vec;    // FP64 v (alpha dot product, extra coordinate)
+  const float* v32;     // FP32 copy of v (mode 0 and 1)
+  const double* vec;    // FP64 v (alpha dot product, extra coordinate); v as pairs (mode 2 and 3)
   const float2* ukin;   // kinetic (hi, lo) pairs
   const float2* ukin_z; // its z part where it is kept apart (one-launch tensor-core kinetic), or null
   const float* rot_hi;  // rotor energies, head and tail
@@ -297,6 +297,7 @@ int fused_update_ctas(const StreamArgs& a, int nn);
 int launch_update_fused(const StreamArgs& a, int nn, int role, cudaStream_t s);
 int launch_vapply_light(const StreamArgs& a, int nn, cudaStream_t s);
 long long vstream_tile_points();
+bool vstream_apart_supported(int vformat, int nn);  // whether there is an apply that adds ukin_z
 // double-float update R = g (R - alpha c V), beta and the next scales, streamed
 // with bulk copies (V, R 16-byte aligned; partials sized for 2 CTAs per SM)
 // j == 0: the iteration is read from *jdev, which the last block then advances

@@ -722,8 +722,11 @@ int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, 
   const long long dpk = N * t.nn;
   if (h->precision == BSL_PREC_MIXED) {
     StreamArgs a = vstream_args(h, v, out);
-    a.vpair = mode == 0 && h->kinetic_engine == BSL_KIN_TENSOR ? d.vpair : nullptr;
     a.mode = mode;
+    if (mode == 0 && h->kinetic_engine == BSL_KIN_TENSOR) {  // v as the pairs that the kinetic reads
+      a.vec = reinterpret_cast<const double*>(d.vpair);
+      a.mode = 3;
+    }
     a.j = j;
     a.defer = mode == 2 ? h->defer_reductions : 0;
     return launch_vapply_f32(a, t.nn, s);

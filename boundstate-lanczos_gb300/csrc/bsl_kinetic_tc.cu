@@ -178,8 +178,25 @@ enum Kinds { kXY = 1, kZ = 2, kAll = 3 };
 // T tiles in shared memory: Z T0 T1 T2 T3 Z of x/y, the slices of Tz, or both
 __host__ __device__ constexpr int t_tiles(int kinds) { return kinds == kXY ? kTS + 2 : kinds == kZ ? kTS : 2 * kTS + 2; }
 
+// After a time-out: NaN in the planes of the CTA's items, so that an H v whose
+// caller does not read the status words (bsl_hv_apply_device) cannot be taken
+// for a result.
 template <int kKinds>
-__device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_stride, int p_end) {
+__device__ __forceinline__ void poison(const KinTC& a) {
+  pdl_wait();
+  const Planes pg{a.nx, a.ny, a.nz, a.nz * a.nn, a.ny * a.nn};
+  for (Items<kKinds> w(pg, blockIdx.x, gridDim.x, 1 << 30); w.more(); w.next())
+    for (int e = threadIdx.x; e < 2 * pg.rows(w.z) * a.nx; e += blockDim.x) {
+      const int row = e / a.nx, pl = row >= pg.rows(w.z), plane = 2 * w.pair + pl;
+      if (plane < pg.count(w.z))
+        (w.z ? a.out_z : a.out_xy)[pg.base(w.z, plane) + (long long)(row - pl * pg.rows(w.z)) * pg.row_stride(w.z) +
+                                   e % a.nx] = make_float2(__int_as_float(0x7fc00000), 0.f);
+    }
+}
+
+// whether the CTA did its items (false after a time-out)
+template <int kKinds>
+__device__ __forceinline__ bool kin_ws_body(const KinTC& a, int p_first, int p_stride, int p_end) {
   extern __shared__ uint8_t smraw[];
   uint8_t* sm = align1024(smraw);
   uint8_t* V = sm + t_tiles(kKinds) * kTile;
@@ -198,7 +215,7 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
   // that the whole CTA takes the same branch
   if (tid == 0) skip = *(volatile int*)(a.status + 3);
   __syncthreads();
-  if (skip) return;
+  if (skip) return false;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -472,11 +489,15 @@ __device__ __forceinline__ void kin_ws_body(const KinTC& a, int p_first, int p_s
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, kStages * kAccCols);
   }
+  return !failed;
 }
 
 template <int kKinds>
-__global__ void __launch_bounds__(kWsThreads, 1) k_kin_tc(KinTC a) {
-  kin_ws_body<kKinds>(a, blockIdx.x, gridDim.x, 1 << 30);
+__global__ void __launch_bounds__(kWsThreads, 1) k_kin_tc(const __grid_constant__ KinTC a) {
+  if (kin_ws_body<kKinds>(a, blockIdx.x, gridDim.x, 1 << 30)) return;
+  const KinTC* again = &a;  // read anew: nothing is kept in registers for a time-out
+  asm volatile("" : "+l"(again));
+  poison<kKinds>(*again);
 }
 
 // Grouped launch over several problems (each with its own grid, T image and
@@ -648,9 +669,20 @@ int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nct
 // against 42.2, 33^3 with 15 35.1 against 38.7, with 21 45.1 against 50.5.
 // Beyond, the z launch's setup is hidden behind the x/y launch's tail and the
 // added bytes are not: 41^3 with 21 62.2 against 58.5 us, 54^3 113 against 88.
+//
+// In a flat box few CTAs have x/y pairs and two launches overlap, and the apply of
+// blocks without the fused iteration hides the added loads worse: 54x54x12 with 10
+// functions 32.5 against 32.0 us (with 9 32.4 against 33.4), 48x48x16 with 16 39.9
+// against 39.4 (30x30x10 31.2 against 33.4), 40x40x10 with 28 52.1 against 49.5 (but 30^3 with 28 54.9 against 56.9 and 40x40x10 with
+// 21 39.1 against 44.1); with 36 functions 70.4 against 64.5 at 40x40x10.
 bool kin_tc_one_launch(const bsl_handle* h) {
-  return h->t.npts * h->t.nn <= 800000;
+  const Tables& t = h->t;
+  if (!h->d.ukin_z || !vstream_apart_supported(h->vformat, t.nn)) return false;
+  if (t.nn <= 9) return true;
+  if (fused_update_supported(h->vformat, t.nn)) return 4 * t.nz >= t.ny;
+  return t.nn <= 16 ? 3 * t.nz > t.ny || t.npts * t.nn <= 400000 : t.nz == t.ny;
 }
+bool kin_tc_small(const Tables& t) { return t.npts * t.nn <= 800000; }
 
 int launch_kin_xy_tc(bsl_handle* h, const float2* v, cudaStream_t s) {
   return kin_tc_one_launch(h) ? launch_kinds<kAll>(h, v, s) : launch_kinds<kXY>(h, v, s);

@@ -92,9 +92,17 @@ __device__ __forceinline__ void bulk_copy_hint(void* dst, const void* src, uint3
 // Blocks of 21-28 functions: the register budget of three resident CTAs per SM
 // (the launcher sizes the grid from the occupancy), which lets the epilogue
 // keep 11 functions' loads in flight (measured: 102.7 instead of 106.1 us per
-// 54^3 iteration, bit-identical); other sizes give no minimum (0) and keep the
-// compiler's choice.
-__host__ __device__ constexpr int vstream_min_ctas(int nn) { return nn >= 21 && nn <= 28 ? 3 : 0; }
+// 54^3 iteration, bit-identical).  36 functions: two CTAs per SM (248 registers, 50.0
+// us at 41x30x20 against 53.7 with the 168 the compiler would take).  Smaller
+// blocks give no minimum (0) and keep the compiler's choice.
+__host__ __device__ constexpr int vstream_min_ctas(int nn) { return nn >= 21 && nn <= 28 ? 3 : nn > 28 ? 2 : 0; }
+// The apply that adds the z part of the kinetic from a buffer of its own, for the
+// FP32 formats.  Whether there is one is fixed at
+// compile time: as a test on each load it cost 2-5 % with 28 and 36 functions, whose
+// registers are the limit, also where there was none.
+__host__ __device__ constexpr bool vstream_apart(int nn, int fmt) {
+  return fmt != 1 && nn <= 28;
+}
 __host__ __device__ constexpr int vstream_load_group(int nn) { return nn >= 21 && nn <= 28 ? 11 : 7; }
 
 // Persistent: CTA b owns the contiguous tiles [b * A.tiles_per_cta, ...), and
@@ -122,7 +130,7 @@ __host__ __device__ constexpr int rows_per_tile() {
 // The CTA's tiles are [t0, t1); it is block `index` of the `count` blocks that
 // reduce alpha together (the grid for one problem; a problem's blocks in a
 // grouped launch).
-template <int NN, int kFmt, int kRole = 0>
+template <int NN, int kFmt, int kRole = 0, bool kApart = false>
 __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, long long t1_arg, unsigned int index,
                                              unsigned int count) {
   constexpr bool kBF = kFmt == 1;
@@ -239,12 +247,12 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       if (kRole == 2) {
         vv[s] = valid ? Vp[s * npts + p].x : 0.f;
         vlo[s] = 0.f;
-      } else if (A.mode == 2) {
+      } else if (A.mode >= 2) {
         const float2 x = valid ? Vp[s * npts + p] : make_float2(0.f, 0.f);
         vv[s] = x.x;
         vlo[s] = x.y;
       } else {
-        vv[s] = !valid ? 0.f : A.vpair ? A.vpair[s * npts + p].x : A.v32[s * npts + p];
+        vv[s] = valid ? A.v32[s * npts + p] : 0.f;
         vlo[s] = 0.f;
       }
       va[s] = 0.f;
@@ -327,7 +335,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
           for (int u = 0; u < kGroup; ++u)
             if (s0 + u < NN) {
               uk[u] = A.ukin[(s0 + u) * npts + p];
-              if (A.ukin_z) uk[u] = df_add_fast(uk[u], A.ukin_z[(s0 + u) * npts + p]);
+              if constexpr (kApart) uk[u] = df_add_fast(uk[u], A.ukin_z[(s0 + u) * npts + p]);
               rr[u] = Rp[(s0 + u) * npts + p];
             }
 #pragma unroll
@@ -347,13 +355,13 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
 #pragma unroll
         for (int s = 0; s < NN; ++s) {
           float2 uk = A.ukin[s * npts + p];
-          if (A.ukin_z) uk = df_add_fast(uk, A.ukin_z[s * npts + p]);
+          if constexpr (kApart) uk = df_add_fast(uk, A.ukin_z[s * npts + p]);
           const float a = fmaf(__ldg(A.rot_hi + s), vv[s], va[s]);
           float hi, e;
           two_sum(uk.x, a, hi, e);
           const float lo = uk.y + e + __ldg(A.rot_lo + s) * vv[s];
           const double hv = f64_of(hi) + f64_of(lo);
-          if (A.mode == 0) {
+          if (A.mode != 1) {
             A.out[s * npts + p] = hv;
           } else {
             const double r = fma(c, hv, A.out[s * npts + p]);
@@ -364,10 +372,9 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       }
     }
   }
-  if (kRole == 0 && A.mode == 0 && (abort_flag || *(volatile int*)(A.status + 3))) {
-    // H v on its own, after a time-out here or in the kinetic: NaN in the CTA's
-    // points, so that a caller who does not read the status words
-    // (bsl_hv_apply_device) cannot take them for a result
+  if (kRole == 0 && abort_flag && (A.mode == 0 || A.mode == 3)) {
+    // H v on its own: NaN in the CTA's points, so that a caller who does not read
+    // the status words (bsl_hv_apply_device) cannot take them for a result
     for (long long p = t0 * kTilePts + tid; p < t1 * kTilePts && p < npts; p += kTilePts)
       for (int s = 0; s < NN; ++s) A.out[s * npts + p] = __longlong_as_double(0x7ff8000000000000ll);
   }
@@ -393,7 +400,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
     }
     return;
   }
-  if (kRole == 0 && A.mode != 0) {
+  if (kRole == 0 && A.mode != 0 && A.mode != 3) {
     // extra coordinate: H acts as 0, R' = R
     if (index == 0 && tid == 0) {
       if (A.mode == 2)
@@ -421,10 +428,10 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
   }
 }
 
-template <int NN, int kFmt, int kRole = 0>
+template <int NN, int kFmt, int kRole = 0, bool kApart = false>
 __global__ void __launch_bounds__(kTilePts, vstream_min_ctas(NN)) k_vstream(const StreamArgs A) {
   const long long t0 = (long long)blockIdx.x * A.tiles_per_cta;
-  vstream_body<NN, kFmt, kRole>(A, t0, t0 + A.tiles_per_cta, blockIdx.x, gridDim.x);
+  vstream_body<NN, kFmt, kRole, kApart>(A, t0, t0 + A.tiles_per_cta, blockIdx.x, gridDim.x);
 }
 
 // The H v apply of a graph-replayed iteration whose block product was formed
@@ -521,27 +528,29 @@ __global__ void __launch_bounds__(kTilePts, 3) k_vstream_group(const StreamArgs*
   }
 }
 
-// the grid of k_vstream<NN, kFmt, kRole> for a (and its tiles per CTA)
-template <int NN, int kFmt, int kRole = 0>
+// the grid of k_vstream<NN, kFmt, kRole, kApart> for a (and its tiles per CTA)
+template <int NN, int kFmt, int kRole = 0, bool kApart = false>
 long long vstream_grid(const StreamArgs& a, long long* tiles_per_cta) {
   const size_t smem = (size_t)kStages * kChunk * kTilePts * sizeof(float);
-  cudaFuncSetAttribute(k_vstream<NN, kFmt, kRole>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_vstream<NN, kFmt, kRole, kApart>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const long long tiles = (a.npts + kTilePts - 1) / kTilePts;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vstream<NN, kFmt, kRole>, kTilePts, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vstream<NN, kFmt, kRole, kApart>, kTilePts, smem);
   if (a.ctas_per_sm > 0 && a.ctas_per_sm < per_sm) per_sm = a.ctas_per_sm;
   const long long slots = (long long)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   *tiles_per_cta = (tiles + slots - 1) / slots;
   return (tiles + *tiles_per_cta - 1) / *tiles_per_cta;
 }
 
-template <int NN, int kFmt = 0, int kRole = 0>
+template <int NN, int kFmt = 0, int kRole = 0, bool kApart = false>
 int launch_nn(StreamArgs a, cudaStream_t s) {
+  if constexpr (kRole == 0 && !kApart && vstream_apart(NN, kFmt))
+    if (a.ukin_z) return launch_nn<NN, kFmt, 0, true>(a, s);
   const size_t smem = (size_t)kStages * kChunk * kTilePts * sizeof(float);
-  const long long grid = vstream_grid<NN, kFmt, kRole>(a, &a.tiles_per_cta);
-  const cudaError_t e = launch_pdl(k_vstream<NN, kFmt, kRole>, dim3((unsigned)grid), dim3(kTilePts), smem, s, a);
+  const long long grid = vstream_grid<NN, kFmt, kRole, kApart>(a, &a.tiles_per_cta);
+  const cudaError_t e = launch_pdl(k_vstream<NN, kFmt, kRole, kApart>, dim3((unsigned)grid), dim3(kTilePts), smem, s, a);
   return e == cudaSuccess ? BSL_OK : cuda_fail(e, "potential stream launch");
 }
 
@@ -778,6 +787,9 @@ int launch_light_group(const void* d_args, const int4* d_work, int nctas, cudaSt
 }
 
 long long vstream_tile_points() { return kTilePts; }
+bool vstream_apart_supported(int vformat, int nn) {
+  return vformat != BSL_VFMT_BF16 && vstream_apart(nn, vformat == BSL_VFMT_GAUNT ? 2 : 0);
+}
 
 // BF16 blocks: tile-major like the FP32 blocks, each point's elements divided
 // by that point's largest |element| (the FP32 scale), rounded to nearest
