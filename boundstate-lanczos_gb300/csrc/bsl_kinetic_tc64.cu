@@ -19,7 +19,7 @@
 //   * the classes from 8 on: 2^-69 root mean square for 64 terms of digits without
 //     a pattern, at most 2^-63;
 //   * the class sums 0-6 are integers below 2^24 and exact (kinetic_smem_image64
-//     refuses a T whose slices could pass that), class 7 is rounded at 2^-71;
+//     refuses a T whose slices could pass that), one unit of class 7 is 2^-79;
 //   * the classes are put together as integers and rounded once.
 // The sum of |T v| along the line is at least 2^-12.7 of the same product, so this
 // stays below one FP64 rounding (2^-53) of that sum, and below a dot product's
@@ -150,28 +150,28 @@ struct Items64 {
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
 
 // What a thread's line scales by: class 3's unit 2^s as 2^b 2^rest, rest 0 unless
-// the products with 2^b could leave the normal range, and -(3 2^51 + 3 2^23) 2^b.
+// the products with 2^b could leave the normal range, and -(3 2^51 + 3 2^15) 2^b.
 struct LineScale {
   int b, rest;
   double unit, shift;
   __device__ __forceinline__ explicit LineScale(int s) : b(min(max(s, -900), 900)) {
     rest = s - b;
     unit = pow2(b);
-    shift = __longlong_as_double((long long)(1023 + b + 52) << 52 | 0x8008000001800000ll);
+    shift = __longlong_as_double((long long)(1023 + b + 52) << 52 | 0x8008000000018000ll);
   }
 };
 
-// (hi + lo 2^-28) 2^b rounded to nearest: hi and lo placed in the mantissas of
-// 3 2^51 + hi and 3 2^23 + lo 2^-28 and added with one rounding.  (The same on the
+// (hi + lo 2^-36) 2^b rounded to nearest: hi and lo placed in the mantissas of
+// 3 2^51 + hi and 3 2^15 + lo 2^-36 and added with one rounding.  (The same on the
 // integer pipe, about 40 operations, is no faster: 386 against 367 us an iteration.)
 __device__ __forceinline__ double rounded(long long hi, long long lo, const LineScale& q) {
-  const double h = __longlong_as_double(hi + (0x4338ll << 48)), l = __longlong_as_double(lo + (0x4178ll << 48));
+  const double h = __longlong_as_double(hi + (0x4338ll << 48)), l = __longlong_as_double(lo + (0x40f8ll << 48));
   return fma(l, q.unit, fma(h, q.unit, q.shift));
 }
 
-// 4 consecutive columns of the eight classes as FP64 values.  Classes 0-3 and 4-7
-// are put together as 64-bit integers, the second in units of 2^-28 of class 3's
-// (class 7 rounded there: 2^-71 of 2^(e + e_t)), and rounded once.
+// 4 consecutive columns of the eight classes as FP64 values: classes 0-3 and 4-7
+// put together as 64-bit integers (below 2^46 and 2^51), the second in units of
+// 2^-36 of the first's, and rounded once.
 __device__ __forceinline__ void combine4(uint32_t taddr, const LineScale& q, double (&out)[4]) {
   float c[kS][4];
 #pragma unroll
@@ -180,9 +180,9 @@ __device__ __forceinline__ void combine4(uint32_t taddr, const LineScale& q, dou
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int c12 = __float2int_rn(c[1][u]) * 512 + __float2int_rn(c[2][u]);
-    const int c67 = __float2int_rn(__fmaf_rn(c[7][u], 0x1p-8f, __fadd_rn(c[6][u], c[6][u])));
     const long long hi = ((long long)__float2int_rn(c[0][u]) << 27) + ((long long)c12 << 9) + __float2int_rn(c[3][u]);
-    const long long lo = ((long long)__float2int_rn(c[4][u]) << 19) + ((long long)__float2int_rn(c[5][u]) << 10) + c67;
+    const long long lo = ((long long)__float2int_rn(c[4][u]) << 27) + ((long long)__float2int_rn(c[5][u]) << 18) +
+                         ((long long)__float2int_rn(c[6][u]) << 9) + __float2int_rn(c[7][u]);
     out[u] = rounded(hi, lo, q);
   }
   for (int rest = q.rest; rest != 0;) {

@@ -63,9 +63,8 @@ def sliced(T, v):
             for l in range(S - k):
                 cls[k + l] += b[l] @ a[k]
         assert np.abs(cls[:7]).max() < 2 ** 24
-        f = cls.astype(np.float32)  # the accumulators; class 7 is rounded to units of 2^-71
-        c67 = np.rint((f[7].astype(np.float64) * 2.0 ** -8 + 2.0 * f[6]).astype(np.float32)).astype(np.int64)
-        out[:, c] = [rounded(sum(int(x) << (55 - 9 * k) for k, x in enumerate(cls[:6, y])) + int(c67[y]), e + et - 71)
+        cls = cls.astype(np.float32).astype(np.int64)  # the accumulators
+        out[:, c] = [rounded(sum(int(x) << (9 * (7 - k)) for k, x in enumerate(cls[:, y])), e + et - 79)
                      for y in range(len(T))]
     return out
 
