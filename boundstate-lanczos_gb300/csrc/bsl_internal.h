@@ -244,6 +244,7 @@ int launch_kin_small(bsl_handle* h, const float2* v, int fin_count, cudaStream_t
 bool kinetic_smem_image64(const std::vector<double>& T, int n, std::vector<uint16_t>* image, int* e_t);
 int launch_kin_tc64(bsl_handle* h, const double* v, bool xy, cudaStream_t s);
 bool kin_f64_tensor(const bsl_handle* h);
+bool kin_f64_one_launch(const bsl_handle* h);
 void kinetic_tc_image(const Tables& t, std::vector<uint16_t>* image, int* tz_tile, int* e_txy, int* e_tz);
 // whether launch_kin_xy_tc forms all three contractions (z in d.ukin_z) and launch_kin_z_tc nothing
 bool kin_tc_one_launch(const bsl_handle* h);

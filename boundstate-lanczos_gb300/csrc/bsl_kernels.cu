@@ -389,7 +389,9 @@ __global__ void k_vblocks(BlockTables bt, const double* v1, const double* v2, lo
 // operations take), so that one launch and no second pass over u_kin remain; T
 // is symmetric and read along its rows by consecutive threads.  13.5 us at 15^3,
 // 21 functions, against 11.4 + 7.4 us for x, y and z in two launches (and one
-// launch less); 27 against 22 + 14 us at 21^3.
+// launch less); 27 against 22 + 14 us at 21^3.  kXYZ false: x and y only, for the
+// grids of kin_f64_one_launch's other side.
+template <bool kXYZ>
 __global__ void k_kin_f64(const double* __restrict__ vec, double* __restrict__ out, const double* __restrict__ tx,
                           const double* __restrict__ ty, const double* __restrict__ tz, int nx, int ny, int nz) {
   extern __shared__ double plane[];
@@ -405,13 +407,36 @@ __global__ void k_kin_f64(const double* __restrict__ vec, double* __restrict__ o
     const double* row = plane + j * nx;
     const double* tyr = ty + (long long)j * ny;
     double ax = 0.0, ay = 0.0, az = 0.0;
+    if (kXYZ)
 #pragma unroll 4
-    for (int q = 0; q < nz; ++q) az += __ldg(tzr + q) * __ldg(col + (long long)q * np);
+      for (int q = 0; q < nz; ++q) az += __ldg(tzr + q) * __ldg(col + (long long)q * np);
 #pragma unroll 4
     for (int q = 0; q < nx; ++q) ax += __ldg(tx + q * nx + i) * row[q];
 #pragma unroll 4
     for (int q = 0; q < ny; ++q) ay += __ldg(tyr + q) * plane[q * nx + i];
-    out[base + e] = az + (ay + ax);
+    out[base + e] = kXYZ ? az + (ay + ax) : ay + ax;
+  }
+}
+
+// z contraction of one (s, j) plane, added: out += Tz.v (the second launch)
+__global__ void k_kin_z_f64(const double* __restrict__ vec, double* __restrict__ out, const double* __restrict__ tz,
+                            int nx, int ny, int nz) {
+  extern __shared__ double plane[];  // [k][i]
+  const int np = nx * nz;
+  const long long sb = (long long)blockIdx.y * nz * ny * nx + (long long)blockIdx.x * nx;
+  for (int e = threadIdx.x; e < np; e += blockDim.x) {
+    const int k = e / nx;
+    plane[e] = vec[sb + (long long)k * ny * nx + (e - k * nx)];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < np; e += blockDim.x) {
+    const int k = e / nx, i = e - k * nx;
+    const double* tr = tz + (long long)k * nz;
+    double az = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < nz; ++q) az += __ldg(tr + q) * plane[q * nx + i];
+    const long long o = sb + (long long)k * ny * nx + i;
+    out[o] = az + out[o];
   }
 }
 
@@ -715,6 +740,12 @@ __global__ void k_ritz_full(const double* __restrict__ ritz, const int* __restri
     o[p] = s >= 0 ? in[p] : masked;
 }
 
+int sm_count(const bsl_handle* h) {
+  int n = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, h->p.device);
+  return n > 0 ? n : 1;
+}
+
 int launch_vapply(bsl_handle* h, const double* v, double* out, int mode, int j, cudaStream_t s) {
   DeviceState& d = h->d;
   const Tables& t = h->t;
@@ -747,19 +778,24 @@ int launch_kin_z(bsl_handle* h, const float2* vpair, cudaStream_t s) {
   return h->kinetic_engine == BSL_KIN_TENSOR ? launch_kin_z_tc(h, vpair, s) : launch_kin_z_mixed(h, h->d.v32, s);
 }
 
-// FP64 kinetic stage: x and y (xy) into d.ukin, or z added to it; without the
-// tensor cores all three in the first stage and nothing in the second
+// FP64 kinetic stage: x and y (xy) into d.ukin, or z added to it; all three in the
+// first stage and nothing in the second where one launch forms them
 int launch_kin_f64(bsl_handle* h, const double* v, bool xy, cudaStream_t s) {
   if (kin_f64_tensor(h)) return launch_kin_tc64(h, v, xy, s);
-  if (!xy) return BSL_OK;
   DeviceState& d = h->d;
   const Tables& t = h->t;
-  const size_t smem = sizeof(double) * t.nx * t.ny;
-  if (smem > 200 * 1024 || sizeof(double) * t.nx * t.nz > 200 * 1024)
-    return fail(BSL_ERR_UNSUPPORTED, "grid plane too large for one CTA");
-  cudaFuncSetAttribute(k_kin_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int threads = std::min(kThreads, (t.nx * t.ny + 31) / 32 * 32);
-  k_kin_f64<<<dim3(t.nz, t.nn), threads, smem, s>>>(v, d.ukin, d.tx, d.ty, d.tz, t.nx, t.ny, t.nz);
+  const size_t sm_xy = sizeof(double) * t.nx * t.ny, sm_z = sizeof(double) * t.nx * t.nz;
+  if (sm_xy > 200 * 1024 || sm_z > 200 * 1024) return fail(BSL_ERR_UNSUPPORTED, "grid plane too large for one CTA");
+  const bool one = kin_f64_one_launch(h);
+  if (xy) {
+    const auto kernel = one ? k_kin_f64<true> : k_kin_f64<false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_xy);
+    const int threads = std::min(kThreads, (t.nx * t.ny + 31) / 32 * 32);
+    kernel<<<dim3(t.nz, t.nn), threads, sm_xy, s>>>(v, d.ukin, d.tx, d.ty, d.tz, t.nx, t.ny, t.nz);
+  } else if (!one) {
+    cudaFuncSetAttribute(k_kin_z_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_z);
+    k_kin_z_f64<<<dim3(t.ny, t.nn), kThreads, sm_z, s>>>(v, d.ukin, d.tz, t.nx, t.ny, t.nz);
+  }
   BSL_CUDA(cudaGetLastError());
   return BSL_OK;
 }
@@ -773,13 +809,33 @@ int launch_kinetic(bsl_handle* h, const double* v, const float2* vpair, cudaStre
 
 }  // namespace
 
-// Whether the FP64 kinetic runs on the tensor cores: from 1.6e7 multiply-adds
-// on, which take the FP64 pipes as long (25 us) as the tensor-core kernels' set-up
-// and one plane pair per SM.  Measured, both contractions, odd l <= 5: 39 against 49
-// us at 21^3 (1.2e7), 62 against 52 us at 24^3 (2.1e7), 993 against 127 us at 54^3.
+// Whether one launch forms the whole plain FP64 kinetic.  Not where its CTAs, one
+// per z plane and function, are large, and already from 1,200 points on where there
+// are fewer of them than SMs (two launches spread z over ny CTAs a function).
+// H v in one launch against two: 15^3 with 15 functions 18.4 against 25 us,
+// 37x29x33 with 10 101 against 107, 54x33x20 with 15 123 against 137; 50x54x52 with
+// 21 1,023 against 1,007, with 1 165 against 142, 54x54x12 with 1 126 against 109.
+bool kin_f64_one_launch(const bsl_handle* h) {
+  const Tables& t = h->t;
+  const int np = t.nx * t.ny;
+  return np <= 1200 || (np <= 2000 && t.nz * t.nn >= sm_count(h));
+}
+
+// Whether the FP64 kinetic runs on the tensor cores, by the microseconds that
+// either engine takes.  The plain sums: their multiply-adds at the FP64 pipes' rate,
+// on as many SMs as there are z planes of all functions.  The tensor cores: a
+// set-up and the items of the fullest CTA (two per x/y plane pair, one per z plane
+// pair, whatever the plane fills of its tile).  H v, plain against tensor cores: 22^3
+// with 21 functions 58 against 60 us, 24^3 66 against 60, 30^3 152 against 106; with 15
+// functions 25^3 54 against 60, 27^3 65 against 62; 14x14x54 with 21 60 against 72,
+// 54x54x12 226 against 88, 54^3 with 1 160 against 52.
 bool kin_f64_tensor(const bsl_handle* h) {
   const Tables& t = h->t;
-  return h->kinetic_engine == BSL_KIN_TENSOR && h->d.kxy_slices64 && (double)t.npts * t.nn * (t.nx + t.ny + t.nz) >= 1.6e7;
+  if (h->kinetic_engine != BSL_KIN_TENSOR || !h->d.kxy_slices64) return false;
+  const long long sms = sm_count(h), pxy = ((long long)t.nz * t.nn + 1) / 2, pz = ((long long)t.ny * t.nn + 1) / 2;
+  const double sums = (double)t.npts * t.nn * (t.nx + t.ny + t.nz) * 1.55e-6;
+  const double plain = sums * std::max(1.0, (double)sms / ((double)t.nz * t.nn));
+  return plain > 5.0 + 4.3 * (double)(2 * ((pxy + sms - 1) / sms) + (pz + sms - 1) / sms);
 }
 
 // ---------------------------------------------------------------------------
@@ -1207,11 +1263,13 @@ const char* dev_stage_name(bsl_handle* h, int i) {
   const bool mixed = h->precision == BSL_PREC_MIXED;
   static const char* n64[4] = {"k_kin_f64", "(in k_kin_f64)", "k_vapply<NN,double>", "k_update_fold"};
   static const char* n64t[2] = {"k_kin_xy_tc64", "k_kin_z_tc64"};
+  static const char* n64p[2] = {"k_kin_f64<x,y>", "k_kin_z_f64"};
   static const char* nmx[4] = {"k_kin_xy_split", "k_kin_z_split", "k_vstream<NN>", "k_update_pair"};
   static const char* nts[2] = {"k_kin_small", "(in k_kin_small)"};
   static const char* ntc[4] = {"k_kin_xy_tc", "k_kin_z_tc", "k_vstream<NN>", "k_update_stream"};
   static const char* nto[2] = {"k_kin_xyz_tc", "(in k_kin_xyz_tc)"};
-  if (!mixed) return i < 2 && kin_f64_tensor(h) ? n64t[i] : n64[i];
+  if (!mixed && i < 2 && kin_f64_tensor(h)) return n64t[i];
+  if (!mixed) return i < 2 && !kin_f64_one_launch(h) ? n64p[i] : n64[i];
   if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_small_supported(h)) return nts[i];
   if (i < 2 && h->kinetic_engine == BSL_KIN_TENSOR && kin_tc_one_launch(h)) return nto[i];
   if (fused_iterations(h) && i >= 2)

@@ -869,7 +869,7 @@ int bsl_launches_per_iteration(const bsl_handle* h) {
   // kinetic in one launch: small problems in mixed precision, FP64 without the tensor cores
   const bool one = h->precision == BSL_PREC_MIXED ? h->kinetic_engine == BSL_KIN_TENSOR &&
                                                         (kin_small_supported(h) || kin_tc_one_launch(h))
-                                                  : !kin_f64_tensor(h);
+                                                  : !kin_f64_tensor(h) && kin_f64_one_launch(h);
   return one ? 3 : 4;
 }
 

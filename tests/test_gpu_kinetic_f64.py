@@ -25,10 +25,15 @@ def bare(bsl, n):
     p.x_max = p.y_max = p.z_max = p.px_max = p.py_max = p.pz_max = 0.08
     p.l_max, p.theta_points, p.phi_points, p.symmetry = 0, 2, 2, bsl.SYM["Even"]
     p.total_mass, p.rotational_constant, p.ceiling_potential = 2.01588, 0.709648713, 18.0
-    h = bsl.Hamiltonian.from_cage(p, np.array([[1e7, 0.0, 0.0]]), np.zeros((1, 3)), q_site=np.zeros(3),
-                                  precision="fp64")
-    assert bsl.lib().bsl_launches_per_iteration(C.c_void_p(h.handle.value)) == 4  # the tensor-core kinetic
-    return h
+    return bsl.Hamiltonian.from_cage(p, np.array([[1e7, 0.0, 0.0]]), np.zeros((1, 3)), q_site=np.zeros(3),
+                                     precision="fp64")
+
+
+def kinetic_kernel(bsl, h):
+    ms, names = (C.c_double * 5)(), (C.c_char_p * 5)()
+    f = bsl.lib().bsl_stage_times
+    assert f(C.c_void_p(h.handle.value), 1, C.cast(ms, C.POINTER(C.c_double)), C.cast(names, C.c_void_p)) == 0
+    return names[0].decode()
 
 
 def vectors(n, rng):
@@ -51,6 +56,7 @@ def vectors(n, rng):
 def test_every_element_is_held_to_its_own_sums(bsl, n):
     h = bare(bsl, n)
     try:
+        assert kinetic_kernel(bsl, h) == "k_kin_xy_tc64"
         rng = np.random.default_rng(n[0])
         t = [sinc_dvr_t(k).astype(np.longdouble) for k in n]
         i = np.stack([rng.integers(0, k, 3000) for k in n], 1)
@@ -98,28 +104,44 @@ def test_an_infinity_reaches_its_own_lines_only(bsl):
         h.close()
 
 
+def check(bsl, h, n, engine, kernel, v):
+    """RMS of H v's error over the terms of its sums; each within n roundings of them."""
+    h.set_kinetic_engine(engine)
+    assert kinetic_kernel(bsl, h) == kernel
+    t = [sinc_dvr_t(k).astype(np.longdouble) for k in n]
+    i = np.random.default_rng(2).integers(0, n, (4000, 3))
+    x, y, z = i.T
+    w = v.astype(np.longdouble)
+    parts = [t[0][x] * w[z, y, :], t[1][y] * w[z, :, x], t[2][z] * w[:, y, x].T]
+    exact, terms = sum(p.sum(1) for p in parts), sum(np.abs(p).sum(1) for p in parts)
+    u = np.zeros(v.size)
+    h.hv(v.ravel(), u)
+    off = np.abs(u.reshape(v.shape)[z, y, x] - exact) / terms
+    assert np.max(off) <= sum(n) * 2.0 ** -53
+    return float(np.sqrt(np.mean(off ** 2)))
+
+
 def test_the_cuda_core_engine_selects_the_plain_sums(bsl):
     """In FP64 as well: the same H v from one kernel and the other, and the tensor
     cores' no further off on average, element by element."""
     n = (57, 57, 57)
     h = bare(bsl, n)
     try:
-        t = [sinc_dvr_t(k).astype(np.longdouble) for k in n]
         v = vectors(n, np.random.default_rng(1))["bound state"]
-        i = np.random.default_rng(2).integers(0, 57, (4000, 3))
-        x, y, z = i.T
-        w = v.astype(np.longdouble)
-        parts = [t[0][x] * w[z, y, :], t[1][y] * w[z, :, x], t[2][z] * w[:, y, x].T]
-        exact, terms = sum(p.sum(1) for p in parts), sum(np.abs(p).sum(1) for p in parts)
-        rms = []
-        for engine, launches in (("simt", 3), ("tensor", 4)):
-            h.set_kinetic_engine(engine)
-            assert bsl.lib().bsl_launches_per_iteration(C.c_void_p(h.handle.value)) == launches
-            u = np.zeros(v.size)
-            h.hv(v.ravel(), u)
-            off = np.abs(u.reshape(v.shape)[z, y, x] - exact) / terms
-            assert np.max(off) <= sum(n) * 2.0 ** -53
-            rms.append(float(np.sqrt(np.mean(off ** 2))))
+        rms = [check(bsl, h, n, *e, v) for e in (("simt", "k_kin_f64<x,y>"), ("tensor", "k_kin_xy_tc64"))]
         assert rms[1] <= rms[0], rms
+    finally:
+        h.close()
+
+
+# planes of 1,190 and of 1,225 points (fewer CTAs than SMs), of 1,980 (160 CTAs), 2,025
+# and 4,096 points; 65 points on an axis
+@pytest.mark.parametrize("n,kernel", [((34, 35, 5), "k_kin_f64"), ((35, 35, 7), "k_kin_f64<x,y>"),
+                                      ((45, 44, 160), "k_kin_f64"), ((45, 45, 160), "k_kin_f64<x,y>"),
+                                      ((64, 64, 2), "k_kin_f64<x,y>"), ((9, 65, 3), "k_kin_f64"), ((2, 2, 65), "k_kin_f64")])
+def test_plain_sums_in_one_launch_and_in_two(bsl, n, kernel):
+    h = bare(bsl, n)
+    try:
+        check(bsl, h, n, "simt", kernel, np.random.default_rng(4).standard_normal(n[::-1]))
     finally:
         h.close()
