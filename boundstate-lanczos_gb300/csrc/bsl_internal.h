@@ -217,6 +217,7 @@ int dev_scatter_full(bsl_handle* h, const double* packed, double* full_accum, cu
 // (previous: the v of the iteration just launched, the buffer roles have
 // flipped), then nj of them added to the vectors
 int ritz_block();
+const double* dev_ritz_vector(const bsl_handle* h, bool previous);
 int dev_ritz_save(bsl_handle* h, double* saved, double* sv, cudaStream_t s, bool previous);
 int dev_ritz_accumulate(bsl_handle* h, const double* saved, const double* sv, int nj, const double* coef,
                         const int* active, int ngood, double* ritz, cudaStream_t s);

@@ -1350,10 +1350,13 @@ int dev_full_step_fused(bsl_handle* h, double* v, double* r, long long L, const 
 
 int ritz_block() { return kRitzBlock; }
 
+const double* dev_ritz_vector(const bsl_handle* h, bool previous) {
+  return (h->lanczos_flip ^ (previous ? 1 : 0)) ? h->d.rvec : h->d.vec;
+}
+
 int dev_ritz_save(bsl_handle* h, double* saved, double* sv, cudaStream_t s, bool previous) {
   const long long L = bsl_packed_size(h) + 1;  // with the coordinate outside the symmetry block
-  const double* V = (h->lanczos_flip ^ (previous ? 1 : 0)) ? h->d.rvec : h->d.vec;
-  k_ritz_save<<<1024, kThreads, 0, s>>>(V, L, h->d.scalars, saved, sv);
+  k_ritz_save<<<1024, kThreads, 0, s>>>(dev_ritz_vector(h, previous), L, h->d.scalars, saved, sv);
   BSL_CUDA(cudaGetLastError());
   return BSL_OK;
 }

@@ -725,6 +725,8 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
   const long long D = bsl_packed_size(h), Df = bsl_basis_size(h), L = D + 1;
   int rc;
   if ((rc = ensure_hist(h, niter)) || (rc = init_state(h, start, seed))) return rc;
+  const bool counted = device_counted_iterations(h);
+  if (counted && (rc = ensure_product_buffer(h))) return rc;
   // coefficient schedule with the reference's cumulative-norm cut-off
   std::vector<double> coef((size_t)niter * ngood);
   std::vector<int> active((size_t)niter * ngood);
@@ -736,36 +738,31 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
       coef[(size_t)(j - 1) * ngood + n] = c;
       active[(size_t)(j - 1) * ngood + n] = (cum[n] < (1. - 1.e-16)) ? 1 : 0;
     }
-  double* dcoef = nullptr;
-  int* dact = nullptr;
-  double *dritz = nullptr, *dsaved = nullptr;
-  double* dfull = nullptr;  // the vectors in the reference layout, as many as the device has room for
-  auto cleanup = [&]() {
-    cudaFree(dcoef);
-    cudaFree(dact);
-    cudaFree(dritz);
-    cudaFree(dsaved);
-    cudaFree(dfull);
-  };
-  // V_j of a block of iterations and their scales; one at a time where memory is short
-  int block = ritz_block();
-  cudaError_t e;
-  if ((e = cudaMalloc(&dcoef, coef.size() * sizeof(double))) != cudaSuccess ||
-      (e = cudaMalloc(&dact, active.size() * sizeof(int))) != cudaSuccess ||
-      (e = cudaMalloc(&dritz, (size_t)ngood * L * sizeof(double))) != cudaSuccess) {
-    cleanup();
-    return fail(BSL_ERR_NOMEM, std::string("Ritz buffers: ") + cudaGetErrorString(e));
-  }
-  while ((e = cudaMalloc(&dsaved, block * ((size_t)L + 1) * sizeof(double))) != cudaSuccess) {
+  // One allocation (each costs up to 0.1 ms a call): the vectors, the V_j of a block
+  // of iterations with their scales, which all vectors in the reference layout
+  // take the place of at the end (one copy: in three, into pages that nothing has
+  // touched, 57 MB took 13 ms instead of 2.6), the coefficients and the flags.
+  // Where the device has no room for that, fewer vectors at a time, single
+  // iterations, and at last nothing beside the vectors: V_j added as it is, the
+  // reference layout put together on the host.
+  const size_t nc = (size_t)niter * ngood, nritz = (size_t)ngood * L;
+  double* dev = nullptr;
+  int block = 0;
+  size_t scratch = 0;
+  cudaError_t e = cudaSuccess;
+  const struct {
+    int block, vectors;
+  } plans[] = {{ritz_block(), ngood}, {ritz_block(), 1}, {1, 1}, {0, 0}};
+  for (const auto& plan : plans) {
+    block = plan.block;
+    scratch = (size_t)std::max(block ? block * (L + 1) : 0, plan.vectors * Df);
+    if ((e = cudaMalloc(&dev, (nritz + scratch + nc + (nc + 1) / 2) * sizeof(double))) == cudaSuccess) break;
     cudaGetLastError();
-    dsaved = nullptr;
-    if (block == 1) {
-      cleanup();
-      return fail(BSL_ERR_NOMEM, std::string("Ritz buffers: ") + cudaGetErrorString(e));
-    }
-    block = 1;
+    dev = nullptr;
   }
-  double* dsv = dsaved + (size_t)block * L;
+  if (!dev) return fail(BSL_ERR_NOMEM, std::string("Ritz buffers: ") + cudaGetErrorString(e));
+  double *dritz = dev, *dsaved = dev + nritz, *dsv = dsaved + (size_t)block * L, *dcoef = dsaved + scratch;
+  int* dact = reinterpret_cast<int*>(dcoef + nc);
   cudaStream_t s = d.stream;
   cudaMemcpyAsync(dcoef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dact, active.data(), active.size() * sizeof(int), cudaMemcpyHostToDevice, s);
@@ -775,45 +772,46 @@ int bsl_ritz_vectors_start(bsl_handle* h, int niter, int start, unsigned long lo
   // fused update), v_j and its scale are complete only once iteration j's x/y
   // kinetic has finished the previous beta, so v_j is taken after iteration j
   // (it is that iteration's V, unchanged by it).
-  const bool counted = device_counted_iterations(h);
-  if (counted && ((rc = ensure_product_buffer(h)) || (rc = dev_set_iteration(h, 1, s)) ||
-                  (rc = dev_begin_iterations(h, s)))) {
-    cleanup();
+  if (counted && ((rc = dev_set_iteration(h, 1, s)) || (rc = dev_begin_iterations(h, s)))) {
+    cudaFree(dev);
     return rc;
   }
   int nj = 0;  // V_j saved since the last accumulation
   for (int j = 1; j <= niter && !rc; ++j) {
     if (counted) rc = dev_lanczos_iteration(h, 0, s);
-    if (!rc) rc = dev_ritz_save(h, dsaved + (size_t)nj * L, dsv + nj, s, counted);
+    const size_t c0 = (size_t)(j - 1) * ngood;
+    if (!rc && !block)
+      rc = dev_ritz_accumulate(h, dev_ritz_vector(h, counted), d.scalars + 4, 1, dcoef + c0, dact + c0, ngood, dritz, s);
+    if (!rc && block) rc = dev_ritz_save(h, dsaved + (size_t)nj * L, dsv + nj, s, counted);
     if (!rc && !counted) rc = dev_lanczos_iteration(h, j, s);
-    if (!rc && (++nj == block || j == niter)) {
-      const size_t c0 = (size_t)(j - nj) * ngood;
-      rc = dev_ritz_accumulate(h, dsaved, dsv, nj, dcoef + c0, dact + c0, ngood, dritz, s);
+    if (!rc && block && (++nj == block || j == niter)) {
+      rc = dev_ritz_accumulate(h, dsaved, dsv, nj, dcoef + c0 - (size_t)(nj - 1) * ngood,
+                               dact + c0 - (size_t)(nj - 1) * ngood, ngood, dritz, s);
       nj = 0;
     }
   }
   if (!rc && counted) rc = dev_finish_iterations(h, s);
-  // the reference layout is put together on the device and copied straight into
-  // the caller's buffer, a few vectors at a time where memory is short
-  cudaFree(dsaved);
-  dsaved = nullptr;
-  int group = ngood;
-  while (!rc && cudaMalloc(&dfull, (size_t)group * Df * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    dfull = nullptr;
-    if (group == 1) rc = fail(BSL_ERR_NOMEM, "Ritz vectors");
-    group = (group + 1) / 2;
-  }
   const double off = (Df > D) ? 1.0 / std::sqrt((double)(Df - D)) : 0.0;
+  const int group = block ? (int)std::min<size_t>(ngood, scratch / Df) : 1;
+  std::vector<double> in(block ? 0 : (size_t)L);
   for (int n0 = 0; n0 < ngood && !rc; n0 += group) {
     const int n = std::min(group, ngood - n0);
-    if ((rc = dev_ritz_full(h, dritz + (size_t)n0 * L, n, off, dfull, s))) break;
-    if ((e = cudaMemcpyAsync(ritz + (size_t)n0 * Df, dfull, (size_t)n * Df * sizeof(double), cudaMemcpyDeviceToHost,
-                             s)) != cudaSuccess)
+    double* out = ritz + (size_t)n0 * Df;
+    const double* from = block ? dsaved : dritz + (size_t)n0 * L;
+    if (block && (rc = dev_ritz_full(h, dritz + (size_t)n0 * L, n, off, dsaved, s))) break;
+    if ((e = cudaMemcpyAsync(block ? out : in.data(), from, (size_t)n * (block ? Df : L) * sizeof(double),
+                             cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (!block && (e = cudaStreamSynchronize(s)) != cudaSuccess)) {
       rc = cuda_fail(e, "Ritz vectors");
+    } else if (!block) {
+      const Tables& t = h->t;
+      std::fill(out, out + Df, in[D] * off);
+      for (int k = 0; k < t.nn; ++k)
+        std::copy_n(in.data() + (size_t)k * t.npts, t.npts, out + (size_t)t.full_of[k] * t.npts);
+    }
   }
   e = cudaStreamSynchronize(s);
-  cleanup();
+  cudaFree(dev);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "Ritz vectors");
   return check_status(h);
