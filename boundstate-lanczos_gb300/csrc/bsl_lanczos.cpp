@@ -32,15 +32,18 @@ int dev_to_pair(double* x, long long n, cudaStream_t s);
 
 int ensure_staging(bsl_handle* h) {
   DeviceState& d = h->d;
-  if (!d.copy_stream) {
-    BSL_CUDA(cudaStreamCreateWithFlags(&d.copy_stream, cudaStreamNonBlocking));
-    BSL_CUDA(cudaEventCreateWithFlags(&d.copy_done, cudaEventDisableTiming));
-    BSL_CUDA(cudaEventCreateWithFlags(&d.vec_in, cudaEventDisableTiming));
+  if (!d.copy_stream) BSL_CUDA(cudaStreamCreateWithFlags(&d.copy_stream, cudaStreamNonBlocking));
+  if (!d.copy_done) BSL_CUDA(cudaEventCreateWithFlags(&d.copy_done, cudaEventDisableTiming));
+  if (!d.vec_in) BSL_CUDA(cudaEventCreateWithFlags(&d.vec_in, cudaEventDisableTiming));
+  for (double** p : {&d.ref_vec, &d.ref_out}) {  // each by itself: an earlier call may have got only the first
+    if (*p) continue;
+    const cudaError_t e = cudaMalloc(p, (size_t)bsl_basis_size(h) * sizeof(double) + 16);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return fail(BSL_ERR_NOMEM, std::string("device allocation failed for staging: ") + cudaGetErrorString(e));
+    }
   }
-  if (d.ref_vec) return BSL_OK;
-  const size_t Df = (size_t)bsl_basis_size(h);
-  BSL_CUDA(cudaMalloc(&d.ref_vec, Df * sizeof(double) + 16));
-  BSL_CUDA(cudaMalloc(&d.ref_out, Df * sizeof(double) + 16));
   return BSL_OK;
 }
 
