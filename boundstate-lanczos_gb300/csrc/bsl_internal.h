@@ -95,8 +95,8 @@ struct DeviceState {
   // FP32 heads fl32(T) and tails fl32(T - head), both stored transposed, for the mixed kernels
   float *kx_head = nullptr, *ky_head = nullptr, *kz_head = nullptr;
   float *kx_band = nullptr, *ky_band = nullptr, *kz_band = nullptr;
-  // fixed-point FP16 slices of T (5 zero-padded 64 x 64 tiles) and their scale
-  // exponents, for the tensor-core kinetic
+  // fixed-point FP16 slices of T (zero-padded 64 x 64 tiles: four of x/y between two
+  // of zeros, then four of z) and their scale exponents, for the tensor-core kinetic
   uint16_t* kin_slices = nullptr;  // of x/y, then of z unless the same (kinetic_tc_image)
   int kin_image16 = 0, kin_tz_tile = 0, e_txy = 0, e_tz = 0;
   float2* ukin_z = nullptr;        // one-launch tensor-core kinetic: the z part (x/y in ukin)
@@ -272,7 +272,7 @@ struct StreamArgs {
   const float2* ukin_z; // its z part where it is kept apart (one-launch tensor-core kinetic), or null
   const float* rot_hi;  // rotor energies, head and tail
   const float* rot_lo;
-  double* out;          // mode 0: u = H v; mode 1: the Lanczos r buffer (r += c H v)
+  double* out;          // mode 0, 3: u = H v; mode 1, 2: the Lanczos r buffer (r += c H v)
   const uint16_t* vb16; // BSL_VFMT_BF16: tile-major BF16 blocks, V = vscale[p] * block
   const float* vscale;
   const float* vc;      // BSL_VFMT_GAUNT: tile-major spherical-harmonic coefficients

@@ -193,14 +193,17 @@ struct Factor {
   float h, l;
 };
 
-// RN(k / RN(sqrt(r2))), the two correctly rounded FP64 operations, in 4 FP64
-// instructions.  The FP64 pipe executes 2 lanes a clock and SM, the FP32 and
+// k / sqrt(r2) as the two FP64 operations give it, in 4 FP64 instructions.  The FP64 pipe executes 2 lanes a clock and SM, the FP32 and
 // integer pipes 128, so the reciprocal root y is refined to ~2^-45 in FP32 (the
 // residual 1 - r2 y0^2 of the hardware's estimate with the error of every
 // product), s0 = r2 y and q0 = k y are formed as FP32 pairs, and all three are put
 // together with integer operations; one FP64 residual each then gives the root
 // and the quotient to ~2^-86 before their final rounding (Markstein, IBM J.
-// Res. Dev. 34, 1990).  Sets bad for r2 outside [2^-60, 2^62).
+// Res. Dev. 34, 1990).  That is the correctly rounded result unless the exact one
+// lies within ~2^-86 of the midpoint of two neighbours, about one rounding in 2^33:
+// then it can be the other neighbour, one unit in the last place of one site's
+// term.  (A grid of 41^3 points, 30 x 60 nodes and 60 sites has 2^35 roundings.)
+// Sets bad for r2 outside [2^-60, 2^62).
 __device__ __forceinline__ double quotient_root(const Factor& f, double r2, bool& bad) {
   const unsigned int hi = (unsigned int)__double2hiint(r2), lo = (unsigned int)__double2loint(r2);
   bad = bad || (hi - 0x3C300000u) >= 0x07A00000u;
@@ -227,7 +230,8 @@ __device__ __forceinline__ double quotient_root(const Factor& f, double r2, bool
 // which leaves 4.3 operations for a squared distance, 4 for the term and 1 to
 // add it, against 29 with one thread per node and the compiler's square root
 // and division: 247 instead of 698 ms at 41^3, 30 x 60 nodes, 60 sites (221 ms
-// at the pipe's rate; 303 ms with the starting root and quotient formed in FP64).  The results are the same bits.
+// at the pipe's rate; 303 ms with the starting root and quotient formed in FP64).  The results are those of the plain operations
+// to within what quotient_root says.
 constexpr int kPhis = 3;
 __global__ void __launch_bounds__(kThreads) k_potential_alavi(AtomSet atoms, const double* xg, const double* yg,
                                                               const double* zg, int nx, int ny, long long npts,

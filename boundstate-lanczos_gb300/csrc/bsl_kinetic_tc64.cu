@@ -30,8 +30,8 @@
 //
 // Why: the FP64 pipe executes 2 lanes a clock and SM, so 3 x 54 multiply-adds
 // per coefficient take 0.85 ms at 54^3 and 21 functions.  Measured there, x/y and
-// z: 104 and 57 us against 656 and 337 us of plain sums in two launches; 38 and
-// 23 us at 27^3.  An item (a plane pair and direction) takes its slicing (11,000
+// z: 97 and 57 us against 656 and 337 us of plain sums in two launches; 36 and 22
+// us at 27^3.  An item (a plane pair and direction) takes its slicing (11,000
 // clocks, integer pipe) and its MMAs (8,000) in turn, since the eight slices leave
 // room for one stage; the epilogue (13,000, FP64 additions and the
 // read-modify-write) runs beside them.
@@ -163,7 +163,8 @@ struct LineScale {
 
 // (hi + lo 2^-36) 2^b rounded to nearest: hi and lo placed in the mantissas of
 // 3 2^51 + hi and 3 2^15 + lo 2^-36 and added with one rounding.  (The same on the
-// integer pipe, about 40 operations, is no faster: 386 against 367 us an iteration.)
+// integer pipe, about 40 operations, is no faster: 386 against 367 us an iteration
+// of 54^3.)
 __device__ __forceinline__ double rounded(long long hi, long long lo, const LineScale& q) {
   const double h = __longlong_as_double(hi + (0x4338ll << 48)), l = __longlong_as_double(lo + (0x40f8ll << 48));
   return fma(l, q.unit, fma(h, q.unit, q.shift));

@@ -12,12 +12,10 @@
 // scales, four 9-bit integers) and the class sums are exact integers in FP32,
 // so u_kin is the same bits.
 //
-// What bounds a small grid is the latency of a launch: below 20^3 the two
-// tensor-core kernels take 6-8 us each whatever their work, most of it set-up
-// (tensor memory, the T image, 128 KiB of zeroed stages).  Here one
-// launch takes their place: an iteration takes 19.1 instead of 29.0 us at 15^3,
-// even l <= 4, and 22.2 instead of 36.9 us at 15^3, odd l <= 5.
-// The column loads and their slicing grow as n per point, which ends the range.
+// What bounds a small grid is the latency of a launch: below 20^3 a tensor-core
+// kernel takes 6-8 us whatever its work, most of it set-up (tensor memory, the T
+// image, 128 KiB of zeroed stages).  The column loads and their slicing grow as n
+// per point, which ends the range (kin_small_supported).
 #include <algorithm>
 
 #include "bsl_device.cuh"
@@ -145,11 +143,14 @@ __global__ void __launch_bounds__(kMaxN * kMaxN + 32) k_kin_small(const SmallArg
 
 }  // namespace
 
-// Up to 16 points per axis (the z column in registers): 18.8 against 29.3 us per
-// iteration at 16^3 even l <= 4, 12.7 against 20.2 us at 6^3 odd l <= 3.  The same
-// kernel with columns of up to 24 points gains 1.1x at 17^3 and loses from 20^3
-// on, where its slicing of whole columns by every plane's CTA costs more than the
-// tensor-core kernels' set-up.
+// Up to 16 points per axis (the z column in registers).  Against the tensor cores'
+// one launch, us: H v at 16^3 with 9, 15, 21 and 36 functions 16.5 against 20.7, 22.7
+// against 24.7, 27.1 against 37.2, 41.2 against 55.5; an iteration at 15^3 with 15
+// and 21 functions 20.1 against 21.4, 23.4 against 35.1, at 10^3 with 10 14.8
+// against 18.5.  At 16^3 the iterations with 9, 10 and 15 functions are the other
+// way round (24.1 against 22.3, 19.1 against 18.9, 21.7 against 20.6); they keep the
+// kernel of their H v.  The same kernel with columns of up to 24 points gains 1.1x
+// at 17^3 against two launches and loses from 20^3 on.
 bool kin_small_supported(const bsl_handle* h) {
   const Tables& t = h->t;
   return h->d.tx_slices32 && h->kin_slices == 4 && t.nx <= kMaxN && t.nz <= kMaxN;

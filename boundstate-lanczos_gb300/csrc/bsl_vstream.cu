@@ -19,6 +19,7 @@
 //   u(s) = ukin(s) + B l(l+1) v(s) + sum_s' V_ss' v(s')   (FP32 block product, FP32-pair sums)
 //   mode 0: out = u (FP64);   mode 1: R += c u (FP64), partial alpha = V . R (deterministic grid reduction);
 //   mode 2: mode 1 with V and R as double-float pairs
+//   mode 3: mode 0 with v as double-float pairs (its heads are the operand)
 //
 // The iterations of a Lanczos run (graph-replayed, the fused iteration) split
 // this differently: the update streams the potential and forms the block
