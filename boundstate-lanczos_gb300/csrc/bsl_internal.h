@@ -266,13 +266,13 @@ int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nct
 // FP32 blocks in the tile-major layout of bsl_vstream.cu (vstream_tile_points() points per tile)
 struct StreamArgs {
   const float* vb;      // tile-major FP32 blocks
-  const float* v32;     // FP32 copy of v (mode 0 and 1)
-  const double* vec;    // FP64 v (alpha dot product, extra coordinate); v as pairs (mode 2 and 3)
+  const float* v32;     // FP32 copy of v (mode 0)
+  const double* vec;    // v as pairs (mode 2 and 3)
   const float2* ukin;   // kinetic (hi, lo) pairs
   const float2* ukin_z; // its z part where it is kept apart (one-launch tensor-core kinetic), or null
   const float* rot_hi;  // rotor energies, head and tail
   const float* rot_lo;
-  double* out;          // mode 0, 3: u = H v; mode 1, 2: the Lanczos r buffer (r += c H v)
+  double* out;          // mode 0, 3: u = H v; mode 2: the Lanczos r buffer (r += c H v)
   const uint16_t* vb16; // BSL_VFMT_BF16: tile-major BF16 blocks, V = vscale[p] * block
   const float* vscale;
   const float* vc;      // BSL_VFMT_GAUNT: tile-major spherical-harmonic coefficients

@@ -17,9 +17,8 @@
 //
 // One thread per grid point of a tile of 128 points:
 //   u(s) = ukin(s) + B l(l+1) v(s) + sum_s' V_ss' v(s')   (FP32 block product, FP32-pair sums)
-//   mode 0: out = u (FP64);   mode 1: R += c u (FP64), partial alpha = V . R (deterministic grid reduction);
-//   mode 2: mode 1 with V and R as double-float pairs
-//   mode 3: mode 0 with v as double-float pairs (its heads are the operand)
+//   mode 0: out = u (FP64);   mode 3: the same with v as double-float pairs (its heads are the operand);
+//   mode 2: R += c u, V and R as double-float pairs, partial alpha = V . R (deterministic grid reduction)
 //
 // The iterations of a Lanczos run (graph-replayed, the fused iteration) split
 // this differently: the update streams the potential and forms the block
@@ -182,9 +181,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
 
   const float2* Vp = reinterpret_cast<const float2*>(A.vec);
   float2* Rp = reinterpret_cast<float2*>(A.out);
-  const double c = A.mode == 1 ? A.scalars[6] : 1.0;
   const float2 cc = reinterpret_cast<const float2*>(A.scalars)[8];  // c as a pair (mode 2)
-  double dot = 0.0;
   float2 dacc = make_float2(0.f, 0.f);
   // role 1: -alpha c from the light apply's block totals (every CTA the same
   // fixed-order sum) and the update's scale g = 2^e
@@ -212,7 +209,6 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       for (int s = 0; s < NN; ++s) {
         asm volatile("prefetch.global.L2 [%0];" ::"l"(A.ukin + s * npts + p));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(A.out + s * npts + p));
-        if (A.mode == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(A.vec + s * npts + p));
       }
     }
     // mode 2 reads the pair of v once: its head is the FP32 copy (the block
@@ -323,9 +319,9 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       continue;
     }
     // u = kinetic pair + B l(l+1) v + V v as an FP32 pair.
-    // mode 1: the logical vectors are v = sv V and r = sr R; r + H v is kept as
-    // sr (R + (sv/sr) H V), so R' = R + c H V and alpha = sv sr (V . R').
-    // mode 2: the same with V and R stored as double-float pairs, all on the FP32 pipe.
+    // mode 2: the logical vectors are v = sv V and r = sr R; r + H v is kept as
+    // sr (R + (sv/sr) H V), so R' = R + c H V and alpha = sv sr (V . R'), V and R
+    // stored as double-float pairs, all on the FP32 pipe.
     if (valid) {
       if (A.mode == 2) {
         constexpr int kGroup = vstream_load_group(NN);  // loads in flight before their arithmetic
@@ -362,13 +358,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
           two_sum(uk.x, a, hi, e);
           const float lo = uk.y + e + __ldg(A.rot_lo + s) * vv[s];
           const double hv = f64_of(hi) + f64_of(lo);
-          if (A.mode != 1) {
-            A.out[s * npts + p] = hv;
-          } else {
-            const double r = fma(c, hv, A.out[s * npts + p]);
-            A.out[s * npts + p] = r;
-            dot = fma(A.vec[s * npts + p], r, dot);
-          }
+          A.out[s * npts + p] = hv;
         }
       }
     }
@@ -404,10 +394,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
   if (kRole == 0 && A.mode != 0 && A.mode != 3) {
     // extra coordinate: H acts as 0, R' = R
     if (index == 0 && tid == 0) {
-      if (A.mode == 2)
-        dacc = df_fma(Vp[A.dpk], Rp[A.dpk], dacc);
-      else
-        dot = fma(A.vec[A.dpk], A.out[A.dpk], dot);
+      dacc = df_fma(Vp[A.dpk], Rp[A.dpk], dacc);
     }
     if (A.defer && A.mode == 2) {  // the update forms alpha from the block totals
       const double bt = block_total_df(dacc);
@@ -418,8 +405,7 @@ __device__ __forceinline__ void vstream_body(const StreamArgs& A, long long t0, 
       return;
     }
     double total;
-    const bool last = A.mode == 2 ? reduce_group_df(dacc, A.partials, A.counter, count, index, &total)
-                                  : reduce_group(dot, A.partials, A.counter, count, index, &total);
+    const bool last = reduce_group_df(dacc, A.partials, A.counter, count, index, &total);
     if (last && threadIdx.x == 0) {
       const double alpha = A.scalars[7] * total;
       A.scalars[0] = alpha;
@@ -888,6 +874,7 @@ int launch_vapply_light(const StreamArgs& a, int nn, cudaStream_t s) {
 }
 
 int launch_vapply_f32(const StreamArgs& a, int nn, cudaStream_t s) {
+  if (a.mode == 1) return fail(BSL_ERR_STATE, "the potential stream updates vectors of double-float pairs");
   if (a.vformat == BSL_VFMT_BF16) {
     if (nn == 15) return launch_nn<15, 1>(a, s);
     if (nn == 21) return launch_nn<21, 1>(a, s);
