@@ -670,17 +670,20 @@ int launch_kin_tc_group(bool xy, const void* d_args, const int4* d_work, int nct
 // Beyond, the z launch's setup is hidden behind the x/y launch's tail and the
 // added bytes are not: 41^3 with 21 62.2 against 58.5 us, 54^3 113 against 88.
 //
-// In a flat box few CTAs have x/y pairs and two launches overlap, and the apply of
-// blocks without the fused iteration hides the added loads worse: 54x54x12 with 10
-// functions 32.5 against 32.0 us (with 9 32.4 against 33.4), 48x48x16 with 16 39.9
-// against 39.4 (30x30x10 31.2 against 33.4), 40x40x10 with 28 52.1 against 49.5 (but 30^3 with 28 54.9 against 56.9 and 40x40x10 with
-// 21 39.1 against 44.1); with 36 functions 70.4 against 64.5 at 40x40x10.
+// Where x/y and z planes differ in number their launches overlap, and the apply of
+// blocks without the fused iteration hides the added loads worse.  An iteration
+// in one launch against two, us: 54x54x12 with 10 functions 32.6 against 31.9 (with 9
+// 31.3 against 33.1), 48x48x16 with 21 49.9 against 46.0 and 27x27x41 45.3 against 44.3
+// (40x40x10 39.5 against 40.6), 48x48x16 with 16 39.8 against 39.2 (30x30x10 30.9
+// against 33.2), 40x40x10 with 28 51.0 against 49.2 (30^3 53.5 against 56.0); with 36
+// functions 70.4 against 64.5 at 40x40x10.
 bool kin_tc_one_launch(const bsl_handle* h) {
   const Tables& t = h->t;
   if (!h->d.ukin_z || !vstream_apart_supported(h->vformat, t.nn)) return false;
-  if (t.nn <= 9) return true;
-  if (fused_update_supported(h->vformat, t.nn)) return 4 * t.nz >= t.ny;
-  return t.nn <= 16 ? 3 * t.nz > t.ny || t.npts * t.nn <= 400000 : t.nz == t.ny;
+  if (t.nn <= 9 || t.nz == t.ny) return true;
+  const long long size = t.npts * t.nn;
+  if (fused_update_supported(h->vformat, t.nn)) return 4 * t.nz >= t.ny && size <= 600000;
+  return t.nn <= 16 && (3 * t.nz > t.ny || size <= 400000);
 }
 bool kin_tc_small(const Tables& t) { return t.npts * t.nn <= 800000; }
 
